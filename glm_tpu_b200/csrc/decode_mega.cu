@@ -314,6 +314,12 @@ __device__ __forceinline__ int mg_pick_ks(int units, int K, bool compat, int max
     return best;
 }
 
+// The compatible split of a projection of `rows16` groups of 16 weight rows (a gate / up pair: 8 + 8) and `units` pairs, as the stand-alone
+// kernels add: all warps (mg_gemv's `mma`), or the split of skinny_bf16_kernel for one row and few outputs.
+__device__ __forceinline__ int mg_split(int rows, int rows16, int units, int K) {
+    return rows > 1 && skinny_mma_takes(rows16) ? SKM_WARPS : mg_pick_ks(units, K, true, 0, 0);
+}
+
 // warp_dot_bf16 (gemv_core.cuh) with U steps of loads issued before their arithmetic: the same products added in the same
 // order, but 2 * U 16-byte loads in flight per lane, which the 16 resident warps of an SM need to keep HBM busy.
 template <int R, int U>
@@ -388,10 +394,23 @@ struct MgUnit {
     const bf16* w1;
 };
 
+// The sums of a unit's two weight rows with the mma inner loop of the stand-alone kernels (the two rows are rows 0 and 1 of the
+// 16-row fragment, the others zero: an output of mma.sync depends on its own row and column only); the first lane gets acc.
+template <int R>
+__device__ __forceinline__ void mg_warp_mma(const MgUnit& m, int K, int rows, int warp, int lane, float (&acc)[2][R]) {
+    const int g = lane >> 2, t = lane & 3;
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    skinny_mma_span<2>(g == 0 ? m.w0 : g == 1 ? m.w1 : nullptr, nullptr, g < rows ? m.x + (int64_t)g * m.xs : nullptr, K, warp, t, c);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[j][r] = __shfl_sync(0xffffffffu, c[r & 1], j * 4 + (r >> 1));
+}
+
 // Units of two weight rows over the whole grid: a team of `ks` warps of one CTA owns a unit, splits K, and its first
-// lane hands the R x 2 sums to `epi(unit, acc)`.
+// lane hands the R x 2 sums to `epi(unit, acc)`.  mma: with mg_warp_mma (ks == SKM_WARPS).
 template <int R, typename Get, typename Epi>
-__device__ __forceinline__ void mg_gemv(int units, int K, int ks, int rows, MgSmall& sm, Get get, Epi epi) {
+__device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int rows, MgSmall& sm, Get get, Epi epi) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tpc = MG_WARPS / ks, team = warp / ks, kpart = warp % ks;
     const int total_teams = gridDim.x * tpc;
@@ -406,12 +425,16 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, int rows, MgSm
             for (int r = 0; r < R; ++r) acc[j][r] = 0.f;
         if (u < units) {
             const MgUnit m = get(u);
-            const bf16* xr[R];
+            if (mma) {
+                mg_warp_mma<R>(m, K, rows, warp, lane, acc);
+            } else {
+                const bf16* xr[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) xr[r] = m.x + (int64_t)(r < rows ? r : 0) * m.xs;
-            const bf16* wp[2] = {m.w0, m.w1};
-            mg_warp_dot<R, (R <= 2 ? 8 : (R <= 4 ? 4 : 2))>(xr, wp, kpart * kspan, (kpart + 1) * kspan, lane, acc);
-            warp_reduce_all<R, 2>(acc);
+                for (int r = 0; r < R; ++r) xr[r] = m.x + (int64_t)(r < rows ? r : 0) * m.xs;
+                const bf16* wp[2] = {m.w0, m.w1};
+                mg_warp_dot<R, (R <= 2 ? 8 : (R <= 4 ? 4 : 2))>(xr, wp, kpart * kspan, (kpart + 1) * kspan, lane, acc);
+                warp_reduce_all<R, 2>(acc);
+            }
         }
         if (ks > 1) {
             __syncthreads();
@@ -616,7 +639,8 @@ template <int R>
 __device__ __forceinline__ void mg_gemv_allreduce(const bf16* x, int64_t xs, const bf16* w, int64_t ws, int N, int K, int rows, bf16* out,
                                                   int64_t os, int channel, const MegaArgs& a, MgSmall& sm) {
     const int units = (N + 1) / 2;
-    const int ks = mg_pick_ks(units, K, true, GLMB_AR_SLICE, 2 * R);
+    const bool mma = rows > 1 && a.comm.world == 1 && skinny_mma_takes((N + 15) / 16);  // the exchange of several GPUs stays with the FMA kernel (glmb_skinny_bf16)
+    const int ks = mma ? SKM_WARPS : mg_pick_ks(units, K, true, GLMB_AR_SLICE, 2 * R);
     const int tpc = MG_WARPS / ks;
     const int total_teams = gridDim.x * tpc;
     const int rounds = (units + total_teams - 1) / total_teams;
@@ -625,7 +649,7 @@ __device__ __forceinline__ void mg_gemv_allreduce(const bf16* x, int64_t xs, con
         if (threadIdx.x == 0 && blockIdx.x == 0) raise_status(a.status, GLMB_STATUS_BAD_SHAPE);
         return;
     }
-    mg_gemv<R>(units, K, ks, rows, sm,
+    mg_gemv<R>(units, K, ks, mma, rows, sm,
                [&](int u) {
                    const int n0 = u * 2;
                    return MgUnit{x, xs, w + (int64_t)n0 * ws, w + (int64_t)min(n0 + 1, N - 1) * ws};
@@ -976,8 +1000,8 @@ __device__ MG_CALL void mg_qkv_a(const MegaArgs& a, const MegaLayer& lw, int lay
                               [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.proj_a, a.proj_stride, rows, p0, cnt, vals); });
             return;
         }
-        const int ks = mg_pick_ks(units, H, compat, 0, 0);
-        mg_gemv<R>(units, H, ks, rows, sm,
+        const int ks = mg_split(rows, (N + 15) / 16, units, H);
+        mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{x_s, H, lw.w_qkv_a + (int64_t)n0 * H, lw.w_qkv_a + (int64_t)min(n0 + 1, N - 1) * H};
@@ -1030,8 +1054,8 @@ __device__ MG_CALL void mg_q_b(const MegaArgs& a, const MegaLayer& lw, int layer
                               [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.q_proj, a.q_stride, rows, p0, cnt, vals); });
             return;
         }
-        const int ks = mg_pick_ks(units, Q, compat, 0, 0);
-        mg_gemv<R>(units, Q, ks, rows, sm,
+        const int ks = mg_split(rows, (N + 15) / 16, units, Q);
+        mg_gemv<R>(units, Q, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{q_s, Q, lw.w_q_b + (int64_t)n0 * Q, lw.w_q_b + (int64_t)min(n0 + 1, N - 1) * Q};
@@ -1157,7 +1181,7 @@ __device__ MG_CALL void mg_vproj(const MegaArgs& a, const MegaLayer& lw, int lay
         const int units = hl * per_head;
         const int ks = mg_pick_ks(per_head * hl, L, compat, 0, 0);
         const int64_t head_rows = (int64_t)(a.nope + vd) * L;
-        mg_gemv<R>(units, L, ks, rows, sm,
+        mg_gemv<R>(units, L, ks, false, rows, sm,
                    [&](int u) {
                        const int h = u / per_head, n0 = (u % per_head) * 2;
                        const bf16* wv = lw.kv_b + h * head_rows + (int64_t)a.nope * L;
@@ -1211,8 +1235,8 @@ __device__ MG_CALL void mg_mlp_a(const MegaArgs& a, const MegaLayer& lw, int lay
                                   });
                 return;
             }
-            const int ks = mg_pick_ks(N, H, compat, 0, 0);
-            mg_gemv<R>(N, H, ks, rows, sm,
+            const int ks = mg_split(rows, (N + 7) / 8, N, H);
+            mg_gemv<R>(N, H, ks, rows > 1 && skinny_mma_takes((N + 7) / 8), rows, sm,
                        [&](int u) { return MgUnit{x_s, H, wg + (int64_t)u * H, wu + (int64_t)u * H}; },
                        [&](int u, int, int, float (&acc)[2][R]) {
 #pragma unroll
@@ -1233,8 +1257,8 @@ __device__ MG_CALL void mg_mlp_a(const MegaArgs& a, const MegaLayer& lw, int lay
                 swiglu(lw.shared_gate, lw.shared_up, a.shared_cols, a.act_shared, a.act_shared_stride);
                 return;
             }
-            const int ks = mg_pick_ks(units, H, compat, 0, 0);
-            mg_gemv<R>(units, H, ks, rows, sm,
+            const int ks = mg_split(rows, (E + 15) / 16, units, H);
+            mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((E + 15) / 16), rows, sm,
                        [&](int u) {
                            const int n0 = u * 2;
                            return MgUnit{x_s, H, lw.router_w + (int64_t)n0 * H, lw.router_w + (int64_t)min(n0 + 1, E - 1) * H};
@@ -1364,8 +1388,8 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
                                   [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.partial, H, rows, p0, cnt, vals); });
                 return;
             }
-            const int ks = mg_pick_ks(units, K, compat, 0, 0);
-            mg_gemv<R>(units, K, ks, rows, sm,
+            const int ks = mg_split(rows, (H + 15) / 16, units, K);
+            mg_gemv<R>(units, K, ks, rows > 1 && skinny_mma_takes((H + 15) / 16), rows, sm,
                        [&](int u) {
                            const int n0 = u * 2;
                            return MgUnit{a.act_shared, a.act_shared_stride, lw.shared_down + (int64_t)n0 * K,
@@ -1518,7 +1542,7 @@ __device__ MG_CALL void mg_head_phase(const MegaArgs& a, int phase, MgSmall& sm,
         bf16* x_s = reinterpret_cast<bf16*>(big);
         mg_norm_rows(a, a.num_layers == 0 ? nullptr : a.update, a.residual_a, a.num_layers == 0, a.final_norm, x_s, nullptr, nullptr, sm);
         const int N = a.vocab_local, units = (N + 1) / 2;
-        const int ks = mg_pick_ks(units, H, COMPAT, 0, 0);
+        const int ks = mg_split(rows, (N + 15) / 16, units, H);
         if (!COMPAT) {
             int nf;
             float* scratch = mg_scratch(big, (size_t)rows * H * 2, &nf);
@@ -1540,7 +1564,7 @@ __device__ MG_CALL void mg_head_phase(const MegaArgs& a, int phase, MgSmall& sm,
         unsigned long long run[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) run[r] = 0ull;
-        mg_gemv<R>(units, H, ks, rows, sm,
+        mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{x_s, H, a.lm_head + (int64_t)n0 * H, a.lm_head + (int64_t)min(n0 + 1, N - 1) * H};

@@ -1,8 +1,8 @@
 // Skinny (1..8 row) weight-streaming projections for decode.
 //
 // With 1-8 live rows every projection of the decode step is bound by streaming the weight matrix from
-// HBM once, so these kernels are organised around 16-byte streaming loads (L1 no-allocate), one warp per
-// output feature (two when that shares the activation registers), fp32 accumulation and a fused epilogue:
+// HBM once, so these kernels are organised around 16-byte streaming loads (L1 no-allocate), 16 output features per CTA on mma.sync (or, for
+// few outputs, batched heads and in-kernel all-reduces, a warp per pair of them with FMAs), fp32 accumulation and a fused epilogue:
 // fp32/bf16 store, SwiGLU of a gate/up pair, or an in-kernel all-reduce over peer memory for K-split
 // (tensor-parallel) projections.  The routed experts' FP8 counterparts are in moe_gemv.cu.
 //
@@ -151,6 +151,74 @@ skinny_bf16_kernel(const bf16* __restrict__ x, int64_t xs, int rows, const bf16*
     }
 }
 
+// ---------------------------------------------------------------------------------------------------
+// The same projection for two to eight rows (one problem, no exchange) with `skinny_mma_span` (gemv_core.cuh): 16 output features per CTA, K
+// split over its warps.
+template <int DEPTH>
+__global__ void __launch_bounds__(SK_THREADS, DEPTH == 4 ? 2 : 3)
+skinny_mma_kernel(const bf16* __restrict__ x, int64_t xs, int rows, const bf16* __restrict__ w, int64_t ws, int N, int K, void* __restrict__ out,
+                  int64_t os, int mode, uint32_t* status, int channel) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int first = blockIdx.x * 16;
+    if ((int64_t)N * K * 2 <= SK_PREFETCH_LIMIT) sk_prefetch_rows(w + (int64_t)first * ws, min(16, N - first), ws, K, 2);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float red[SK_WARPS][8 * SKM_RED];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
+    const int n_lo = first + g;
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    skinny_mma_span<DEPTH>(n_lo < N ? w + (int64_t)n_lo * ws : nullptr, n_lo + 8 < N ? w + (int64_t)(n_lo + 8) * ws : nullptr,
+                           g < rows ? x + (int64_t)g * xs : nullptr, K, warp, lane & 3, c);
+    skm_store_fragment(red[warp], c, lane);
+    __syncthreads();
+    if (threadIdx.x >= 128) return;
+    const int r = threadIdx.x >> 4, n = first + (threadIdx.x & 15);
+    const float v = skm_sum(red, r, threadIdx.x & 15);
+    const bool live = n < N && r < rows;
+    if (mode == SK_OUT_ARGMAX || mode == SK_OUT_ARGMAX_F32) {  // see skinny_bf16_kernel
+        unsigned long long key = 0ull;
+        if (live) {
+            const float logit = mode == SK_OUT_ARGMAX ? bf16_round(v) : v;
+            if (!isfinite(logit)) raise_status(status, GLMB_STATUS_NONFINITE);
+            key = candidate_key(logit, channel + n);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
+            key = other > key ? other : key;
+        }
+        if ((lane & 15) == 0 && key) atomicMax(reinterpret_cast<unsigned long long*>(out) + r, key);
+    } else if (live) {
+        if (mode == SK_OUT_F32) reinterpret_cast<float*>(out)[(int64_t)r * os + n] = v;
+        else reinterpret_cast<bf16*>(out)[(int64_t)r * os + n] = __float2bfloat16_rn(v);
+    }
+}
+
+// Gate row n and up row n are rows g and g + 8 of the same fragment: eight outputs per CTA.
+template <int DEPTH>
+__global__ void __launch_bounds__(SK_THREADS, DEPTH == 4 ? 2 : 3)
+skinny_mma_swiglu_kernel(const bf16* __restrict__ x, int64_t xs, int rows, const bf16* __restrict__ wg, const bf16* __restrict__ wu, int64_t ws, int N,
+                         int K, bf16* __restrict__ act, int64_t as) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int first = blockIdx.x * 8;
+    if ((int64_t)N * K * 4 <= SK_PREFETCH_LIMIT) {
+        sk_prefetch_rows(wg + (int64_t)first * ws, min(8, N - first), ws, K, 2);
+        sk_prefetch_rows(wu + (int64_t)first * ws, min(8, N - first), ws, K, 2);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float red[SK_WARPS][8 * SKM_RED];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
+    const int own = first + g;
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    skinny_mma_span<DEPTH>(own < N ? wg + (int64_t)own * ws : nullptr, own < N ? wu + (int64_t)own * ws : nullptr,
+                           g < rows ? x + (int64_t)g * xs : nullptr, K, warp, lane & 3, c);
+    skm_store_fragment(red[warp], c, lane);
+    __syncthreads();
+    const int r = threadIdx.x >> 3, j = threadIdx.x & 7, n = first + j;
+    if (threadIdx.x >= 64 || n >= N || r >= rows) return;
+    const float gv = bf16_round(skm_sum(red, r, j)), uv = bf16_round(skm_sum(red, r, j + 8));
+    act[(int64_t)r * as + n] = __float2bfloat16_rn(gv * sigmoidf_precise(gv) * uv);
+}
+
 // act[r][n] = bf16( silu(bf16(x.w_gate[n])) * bf16(x.w_up[n]) )       (bf16 weights; dense MLP / shared expert)
 template <int R>
 __global__ void __launch_bounds__(SK_THREADS)
@@ -224,8 +292,18 @@ GLMB_API int glmb_skinny_bf16(const void* x, int64_t xs, int rows, const void* w
                               int mode, int batch, int64_t xb, int64_t wb, int64_t ob, const PeerComm* comm, int channel,
                               void* stream) {
     if (rows < 1 || rows > GLMB_MAX_ROWS || (K & 7) || (xs & 7) || (ws & 7) || (xb & 7) || (wb & 7) || batch < 1) return 1;
-    int ks = pick_ksplit(ceil_div(N, 2) * batch, K);
     PeerComm c = comm ? *comm : single_comm();
+    const int groups = ceil_div(N, 16);
+    if (rows > 1 && skinny_mma_takes(groups) && batch == 1 && !(mode == SK_OUT_ALLREDUCE_BF16 && c.world > 1)) {
+#define CALL(D)                                                                                                                            \
+    GLMB_LAUNCH(skinny_mma_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)w, ws, N, K, out, os, mode, \
+                c.status, channel)
+        if (skinny_mma_depth(groups, K) == 4) CALL(4);
+        else CALL(2);
+#undef CALL
+        return (int)cudaGetLastError();
+    }
+    int ks = pick_ksplit(ceil_div(N, 2) * batch, K);
     // A CTA that all-reduces waits for the same CTA of every peer before it retires.  CTAs beyond the first wave would start only
     // after such a wait and then wait again: keep the grid within one wave (three CTAs per SM fit whatever the row count).
     if (mode == SK_OUT_ALLREDUCE_BF16 && c.world > 1)
@@ -244,6 +322,16 @@ GLMB_API int glmb_skinny_bf16(const void* x, int64_t xs, int rows, const void* w
 GLMB_API int glmb_skinny_bf16_swiglu(const void* x, int64_t xs, int rows, const void* wg, const void* wu, int64_t ws, int N, int K,
                                      void* act, int64_t as, void* stream) {
     if (rows < 1 || rows > GLMB_MAX_ROWS || (K & 7) || (xs & 7) || (ws & 7)) return 1;
+    const int groups = ceil_div(N, 8);
+    if (rows > 1 && skinny_mma_takes(groups)) {
+#define CALL(D)                                                                                                                                   \
+    GLMB_LAUNCH(skinny_mma_swiglu_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)wg, (const bf16*)wu, ws, \
+                N, K, (bf16*)act, as)
+        if (skinny_mma_depth(groups, K) == 4) CALL(4);
+        else CALL(2);
+#undef CALL
+        return (int)cudaGetLastError();
+    }
     const int ks = pick_ksplit(N, K);
     const int grid = ceil_div(N, SK_WARPS / ks);
 #define CALL(RR)                                                                                                          \

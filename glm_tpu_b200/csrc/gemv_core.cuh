@@ -1,10 +1,13 @@
 // Per-warp inner loops of the weight-streaming (1..8 row) projections, shared by the stand-alone skinny kernels
-// (gemv.cu) and the persistent decode kernel (decode_mega.cu).  A warp owns NPW weight rows over a K range: every
-// lane streams 16-byte pieces (L1 no-allocate), multiplies them with the R activation rows in fp32 and the warp
-// reduces with the xor tree of warp_sum, so every caller gets the same bits for the same (rows, K range).
+// (gemv.cu, parallel_block.cu, moe_rows.cu) and the persistent decode kernel (decode_mega.cu).
+//
+// `warp_dot_*`: a warp owns NPW weight rows over a K range: every lane streams 16-byte pieces (L1 no-allocate), multiplies them
+// with the R activation rows in fp32 and the warp reduces with the xor tree of warp_sum, so every caller gets the same bits for the
+// same (rows, K range).  `skinny_mma_*`: 16 weight rows on mma.sync, for two to eight rows and all but few outputs.
 #pragma once
 
 #include "common.cuh"
+#include "moe_mma_core.cuh"
 
 // ---------------------------------------------------------------------------------------------------
 // Per-warp dot products.  acc[j][r] accumulates this lane's share of  sum_k w_j[k] * x_r[k].
@@ -75,3 +78,71 @@ __device__ __forceinline__ void warp_reduce_all(float (&acc)[NPW][R]) {
         for (int r = 0; r < R; ++r) acc[j][r] = warp_sum(acc[j][r]);
 }
 
+// ---------------------------------------------------------------------------------------------------
+// 16 weight rows as the M and one to eight activation rows as the N of mma.sync m16n8k16 (bf16 products, fp32 sums).  With R rows the
+// FMA loop above issues R + 2 instructions per weight and is bound by issue from four rows on; here a weight costs a sixteenth of an
+// instruction whatever R is, and nothing is shuffled at the end.  Measured on a B200, [6144 x 16384]: 2 rows 49.8 -> 32.2 us, 4 rows
+// 58.0 -> 32.6, 8 rows 85.5 -> 32.9 (6.1 TB/s); [131072 x 4096]: 193 -> 154, 218 -> 158, 397 -> 163.
+//
+// The k index inside an instruction is a permutation of the true k, the same for both operands: lane (g, t) holds 16 consecutive
+// k values of weight rows g (w_lo) and g + 8 (w_hi) and of activation row g, at 16 t of a 64-wide chunk, so every load is a full
+// 16-byte vector.  Chunks first, first + stride, .. enter the sum in ascending order, whatever DEPTH (chunks whose loads are in
+// flight together) is.  `skinny_mma_span`: the SKM_WARPS warps of a CTA take the chunks of K round-robin; the bits depend on K only.
+// w_lo, w_hi, xr: this lane's rows (NULL: zeros).  K a multiple of 8.  c: the C fragment, rows g and g + 8, columns 2t and 2t + 1.
+#define SKM_WARPS 8
+template <int DEPTH>
+__device__ __forceinline__ void skinny_mma_chunks(const bf16* w_lo, const bf16* w_hi, const bf16* xr, int K, int first, int stride, int chunks, int t,
+                                                  float (&c)[4]) {
+    for (int c0 = first; c0 < chunks; c0 += stride * DEPTH) {
+        uint4 lo[DEPTH][2], hi[DEPTH][2], x[DEPTH][2];
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = ((c0 + u * stride) << 6) + t * 16 + h * 8;
+                const uint4 zero = make_uint4(0, 0, 0, 0);
+                lo[u][h] = w_lo && k < K ? ld_stream16(w_lo + k) : zero;
+                hi[u][h] = w_hi && k < K ? ld_stream16(w_hi + k) : zero;
+                x[u][h] = xr && k < K ? ld_hot16(xr + k) : zero;
+            }
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                mma_16816(c, lo[u][h].x, hi[u][h].x, lo[u][h].y, hi[u][h].y, x[u][h].x, x[u][h].y);
+                mma_16816(c, lo[u][h].z, hi[u][h].z, lo[u][h].w, hi[u][h].w, x[u][h].z, x[u][h].w);
+            }
+    }
+}
+template <int DEPTH>
+__device__ __forceinline__ void skinny_mma_span(const bf16* w_lo, const bf16* w_hi, const bf16* xr, int K, int warp, int t, float (&c)[4]) {
+    skinny_mma_chunks<DEPTH>(w_lo, w_hi, xr, K, warp, SKM_WARPS, (K + 63) >> 6, t, c);
+}
+
+// Whether a projection of so many groups of 16 weight rows takes the kernels above: a CTA has one group, and fewer than 64 CTAs leave the
+// machine idle ([256 x 6144]: 16 CTAs 4.8 us, the FMA kernel's 128 CTAs of two rows 3.1; [2048 x 2048]: 3.8 against 4.4).
+__host__ __device__ static inline bool skinny_mma_takes(int groups) { return groups >= 64; }
+
+// Chunks in flight per warp: four with two CTAs per SM, or two with three.  The last wave decides: whichever fills its waves better ([4096 x
+// 18432], 256 CTAs: 25.4 against 28.0 us; [6144 x 16384], 384 CTAs: 37.4 against 32.6).  Rows of fewer than two rounds of
+// four chunks gain nothing from the deeper form beyond the first wave.
+static inline int skinny_mma_depth(int groups, int K) {
+    if (groups <= 2 * 148) return 4;
+    const int full4 = (groups + 295) / 296 * 296, full2 = (groups + 443) / 444 * 444;
+    return K >= 4096 && full4 < full2 ? 4 : 2;
+}
+
+// Fragments of a CTA's warps meet in shared memory, [column][row] with a stride of 20 floats (no bank conflict on the way in).
+#define SKM_RED 20
+__device__ __forceinline__ void skm_store_fragment(float* red, const float (&c)[4], int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    red[(2 * t) * SKM_RED + g] = c[0]; red[(2 * t + 1) * SKM_RED + g] = c[1];
+    red[(2 * t) * SKM_RED + g + 8] = c[2]; red[(2 * t + 1) * SKM_RED + g + 8] = c[3];
+}
+// Sum over the warps' K parts of (activation row r, weight row n), in warp order.
+__device__ __forceinline__ float skm_sum(const float (*red)[8 * SKM_RED], int r, int n) {
+    float s = red[0][r * SKM_RED + n];
+#pragma unroll
+    for (int p = 1; p < SKM_WARPS; ++p) s += red[p][r * SKM_RED + n];
+    return s;
+}
