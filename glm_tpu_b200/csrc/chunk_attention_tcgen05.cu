@@ -12,8 +12,8 @@
 // output in TMEM is rescaled rarely.
 //
 //   warps 0-3, 4-7   softmax and output of tile 0 and tile 1 (warp w reads TMEM lanes 32 (w % 4) ..)
-//   warp 8           issues every tcgen05.mma (one lane), owns the TMEM allocation
-//   warp 9           TMA producer (one lane): query tiles once, then K and V blocks through two-stage rings
+//   warp 8           issues every tcgen05.mma, owns the TMEM allocation
+//   warp 9           TMA producer: query tiles once, then K and V blocks through two-stage rings
 //
 // Every wait is bounded; a wait that runs out raises GLMB_STATUS_WAIT_TIMEOUT and the CTA still releases its TMEM.
 #include "chunk_attention.cuh"
@@ -35,14 +35,6 @@ __device__ __forceinline__ void fa_tmem_ld32_nowait(uint32_t taddr, uint32_t* r)
           "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void fa_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void fa_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -78,7 +70,7 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     __shared__ __align__(8) uint64_t q_full[2], k_full[FA_STAGES], k_empty[FA_STAGES], v_full[FA_STAGES], v_empty[FA_STAGES], s_full[2], p_full[2], o_full[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t fail;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int kboxes = (a.dimp + 63) / 64, vboxes = (a.vdimp + 63) / 64;
     unsigned char* q_s = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* k_s = q_s + 2 * kboxes * FA_BOX;
@@ -114,58 +106,75 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     const int blocks = max(range[0].end, range[1].end);
 
     if (warp == 9) {
-        if (lane == 0) {
+        if (elect_one())
             for (int t = 0; t < 2; ++t)
                 if (range[t].rows) {
                     mbar_expect_tx(q_full + t, kboxes * FA_BOX);
                     for (int b = 0; b < kboxes; ++b)
                         tma_load_2d(q_s + (t * kboxes + b) * FA_BOX, &map_q, q_full + t, head * a.dimp + b * 64, r0 + t * FA_TILE);
                 }
-            for (int j = 0; j < blocks; ++j) {
-                const int s = j % FA_STAGES, lap = j / FA_STAGES, y = key0 - a.base + j * FA_TILE;
-                if (lap > 0 && !mbar_wait(k_empty + s, (lap - 1) & 1)) { fail = 1; break; }
+        __syncwarp();
+        for (int j = 0; j < blocks; ++j) {
+            const int s = j % FA_STAGES, lap = j / FA_STAGES, y = key0 - a.base + j * FA_TILE;
+            if (lap > 0 && !mbar_wait_warp(k_empty + s, (lap - 1) & 1)) { fail = 1; break; }
+            if (elect_one()) {
                 mbar_expect_tx(k_full + s, kboxes * FA_BOX);
                 for (int b = 0; b < kboxes; ++b) tma_load_2d(k_s + (s * kboxes + b) * FA_BOX, &map_k, k_full + s, group * a.dimp + b * 64, y);
-                if (lap > 0 && !mbar_wait(v_empty + s, (lap - 1) & 1)) { fail = 1; break; }
+            }
+            __syncwarp();
+            if (lap > 0 && !mbar_wait_warp(v_empty + s, (lap - 1) & 1)) { fail = 1; break; }
+            if (elect_one()) {
                 mbar_expect_tx(v_full + s, vboxes * FA_BOX);
                 for (int b = 0; b < vboxes; ++b) tma_load_2d(v_s + (s * vboxes + b) * FA_BOX, &map_v, v_full + s, group * a.vdimp + b * 64, y);
             }
+            __syncwarp();
         }
     } else if (warp == 8) {
-        if (lane == 0) {
-            const uint32_t idesc_s = umma_idesc_bf16(FA_TILE, FA_TILE), idesc_o = umma_idesc_bf16(FA_TILE, a.vdimp) | (1u << 16);  // bit 16: B is MN-major
-            int done[2] = {0, 0};
-            bool ok = true;
-            for (int j = -1; j < blocks && ok; ++j) {
-                for (int t = 0; t < 2 && ok; ++t) {
-                    if (j >= range[t].begin && j < range[t].end) {  // O_t += P_t V_j
-                        if (!mbar_wait(p_full + t, done[t] & 1) || !mbar_wait(v_full + j % FA_STAGES, (j / FA_STAGES) & 1) || fail) { fail = 1; ok = false; break; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t v_addr = smem_u32(v_s + (j % FA_STAGES) * vboxes * FA_BOX);
+        const uint32_t idesc_s = umma_idesc_bf16(FA_TILE, FA_TILE), idesc_o = umma_idesc_bf16(FA_TILE, a.vdimp) | (1u << 16);  // bit 16: B is MN-major
+        int done[2] = {0, 0};
+        bool ok = true;
+        for (int j = -1; j < blocks && ok; ++j) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                if (ok && j >= range[t].begin && j < range[t].end) {  // O_t += P_t V_j
+                    ok = mbar_wait_warp(p_full + t, done[t] & 1) && mbar_wait_warp(v_full + j % FA_STAGES, (j / FA_STAGES) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t v_addr = smem_u32(v_s + (j % FA_STAGES) * vboxes * FA_BOX);
+                    if (elect_one()) {
+#pragma unroll
                         for (int piece = 0; piece < 2; ++piece)
 #pragma unroll
                             for (int k = 0; k < FA_TILE / 16; ++k)
                                 fa_mma_ts(tmem + 256 + t * 128, tmem + t * 128 + piece * 64 + k * 8, fa_desc_mn(v_addr + k * 2048), idesc_o,
                                           (done[t] > 0 || piece > 0 || k > 0) ? 1u : 0u);
-                        ++done[t];
                         if (j + 1 == range[t].end) umma_commit(o_full + t);
                     }
-                    if (j + 1 >= range[t].begin && j + 1 < range[t].end) {  // S_t = Q_t K_{j+1}^T
-                        const int n = j + 1, s = n % FA_STAGES;
-                        if ((n == range[t].begin && !mbar_wait(q_full + t, 0)) || !mbar_wait(k_full + s, (n / FA_STAGES) & 1) || fail) { fail = 1; ok = false; break; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t q_addr = smem_u32(q_s + t * kboxes * FA_BOX), k_addr = smem_u32(k_s + s * kboxes * FA_BOX);
+                    __syncwarp();
+                    ++done[t];
+                }
+                if (ok && j + 1 >= range[t].begin && j + 1 < range[t].end) {  // S_t = Q_t K_{j+1}^T
+                    const int n = j + 1, s = n % FA_STAGES;
+                    ok = (n > range[t].begin || mbar_wait_warp(q_full + t, 0)) && mbar_wait_warp(k_full + s, (n / FA_STAGES) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t q_addr = smem_u32(q_s + t * kboxes * FA_BOX), k_addr = smem_u32(k_s + s * kboxes * FA_BOX);
+                    if (elect_one()) {
                         for (int k = 0; k < a.dimp / 16; ++k) {
                             const uint32_t at = (k >> 2) * FA_BOX + (k & 3) * 32;
                             umma_bf16(tmem + t * 128, umma_desc_sw128(q_addr + at), umma_desc_sw128(k_addr + at), idesc_s, k > 0 ? 1u : 0u);
                         }
                         umma_commit(s_full + t);
                     }
+                    __syncwarp();
                 }
-                if (!ok) break;
+            }
+            if (!ok) { fail = 1; break; }
+            if (elect_one()) {
                 if (j >= 0) umma_commit(v_empty + j % FA_STAGES);            // the blocks may be replaced once these products have read them
                 if (j + 1 < blocks) umma_commit(k_empty + (j + 1) % FA_STAGES);
             }
+            __syncwarp();
         }
     } else {
         const int t = warp >> 2, quarter = warp & 3;
@@ -205,7 +214,7 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 l *= fix;
                 for (int c = 0; c < a.vdimp; c += 16) {
                     uint32_t o[16];
-                    fa_tmem_ld16(o_addr + c, o);
+                    tmem_ld16(o_addr + c, o);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fix);
                     fa_tmem_st16(o_addr + c, o);
@@ -249,7 +258,7 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 const bool vec = !(reinterpret_cast<uintptr_t>(dst) & 15);
                 for (int c = 0; c < a.vdimp; c += 16) {
                     uint32_t o[16];
-                    fa_tmem_ld16(o_addr + c, o);
+                    tmem_ld16(o_addr + c, o);
                     if (row >= range[t].rows) continue;
                     uint32_t w[8];
 #pragma unroll

@@ -5,8 +5,8 @@
 // thread issues tcgen05.mma (kind::f16, bf16 inputs, fp32 accumulate) into a 128-lane x 128-column TMEM
 // accumulator; four epilogue warps read it back with tcgen05.ld, round to bf16 (or keep fp32) and store.
 //
-//   warp 0      TMA producer (one elected lane)
-//   warp 1      TMEM allocation, MMA issue (one elected lane), TMEM release
+//   warp 0      TMA producer (an elected lane issues)
+//   warp 1      TMEM allocation, MMA issue (an elected lane), TMEM release
 //   warps 2-5   epilogue: warp w owns TMEM lanes 32*(w%4) .. +31
 //
 // Grouped mode (routed experts in prefill): `tiles` lists (first row, end row, expert) per 128-row tile of the
@@ -49,7 +49,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
     uint32_t* fail_slot = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int t = blockIdx.y;
     if (n_tiles && t >= *n_tiles) return;
     int row0, row_end, expert;
@@ -74,27 +74,27 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            for (int kb = 0; kb < kblocks; ++kb) {
-                const int s = kb % TC_STAGES;
-                if (kb >= TC_STAGES && !mbar_wait(empty_bar + s, ((kb / TC_STAGES) - 1) & 1)) { *fail_slot = 1; break; }
-                unsigned char* a_dst = ring + s * TC_STAGE_BYTES;
-                unsigned char* b_dst = a_dst + TC_BM * TC_BK * 2;
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const int s = kb % TC_STAGES;
+            if (kb >= TC_STAGES && !mbar_wait_warp(empty_bar + s, ((kb / TC_STAGES) - 1) & 1)) { *fail_slot = 1; break; }
+            unsigned char* a_dst = ring + s * TC_STAGE_BYTES;
+            unsigned char* b_dst = a_dst + TC_BM * TC_BK * 2;
+            if (elect_one()) {
                 mbar_expect_tx(full_bar + s, TC_STAGE_BYTES);
                 tma_load_2d(a_dst, &map_a, full_bar + s, kb * TC_BK, row0);
                 tma_load_2d(b_dst, &map_b, full_bar + s, kb * TC_BK, expert * N + n0);
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, TC_BN);
-            bool ok = true;
-            for (int kb = 0; kb < kblocks && ok; ++kb) {
-                const int s = kb % TC_STAGES;
-                if (!mbar_wait(full_bar + s, (kb / TC_STAGES) & 1)) { *fail_slot = 1; ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = smem_u32(ring + s * TC_STAGE_BYTES);
-                const uint32_t b_addr = a_addr + TC_BM * TC_BK * 2;
+        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, TC_BN);
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const int s = kb % TC_STAGES;
+            if (!mbar_wait_warp(full_bar + s, (kb / TC_STAGES) & 1)) { *fail_slot = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = smem_u32(ring + s * TC_STAGE_BYTES);
+            const uint32_t b_addr = a_addr + TC_BM * TC_BK * 2;
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {
                     const uint64_t da = umma_desc_sw128(a_addr + k * TC_UMMA_K * 2);
@@ -103,8 +103,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 }
                 umma_commit(empty_bar + s);  // the stage may be refilled once these MMAs have read it
             }
-            umma_commit(acc_bar);            // accumulator complete (or abandoned): release the epilogue
+            __syncwarp();
         }
+        if (elect_one()) umma_commit(acc_bar);  // accumulator complete (or abandoned): release the epilogue
+        __syncwarp();
     } else {
         // epilogue
         const int quarter = warp & 3;
@@ -207,7 +209,7 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     volatile uint32_t* fail_slot = tmem_slot + 1;
     unsigned char* epi_stage = ring + T2_STAGES * T2_STAGE_BYTES + 256;  // per epilogue warp: fp32 tile, then bf16 tile
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // every CTA reads the round number before any CTA can finish, and the last CTA to finish advances it
     const uint32_t ar_epoch = ar.enabled ? ar.comm.seq[GLMB_SEQ_GEMM] + 1 : 0;
     const int m_tiles = tiles ? min(max(*n_tiles, 0), max_tiles) : (rows + TC_BM - 1) / TC_BM;
@@ -231,49 +233,53 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t g = 0;  // k-blocks issued so far, across tiles
-            for (int t = blockIdx.x; t < total && !*fail_slot; t += gridDim.x) {
-                int m, n;
-                t2_tile(t, m_tiles, n_blocks, m, n);
-                const int row0 = tiles ? tiles[m].row0 : m * TC_BM;
-                const int b_row = (tiles ? tiles[m].expert : 0) * N + n * T2_BN;
-                for (int kb = 0; kb < kblocks; ++kb, ++g) {
-                    const uint32_t s = g % T2_STAGES, lap = g / T2_STAGES;
-                    if (lap > 0 && !mbar_wait(empty_bar + s, (lap - 1) & 1)) { *fail_slot = 1; break; }
-                    unsigned char* a_dst = ring + s * T2_STAGE_BYTES;
-                    unsigned char* b_dst = a_dst + TC_BM * TC_BK * 2;
+        uint32_t g = 0;  // k-blocks issued so far, across tiles
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            int m, n;
+            t2_tile(t, m_tiles, n_blocks, m, n);
+            const int row0 = tiles ? tiles[m].row0 : m * TC_BM;
+            const int b_row = (tiles ? tiles[m].expert : 0) * N + n * T2_BN;
+            for (int kb = 0; kb < kblocks; ++kb, ++g) {
+                const uint32_t s = g % T2_STAGES, lap = g / T2_STAGES;
+                if (lap > 0 && !mbar_wait_warp(empty_bar + s, (lap - 1) & 1)) { *fail_slot = 1; ok = false; break; }
+                unsigned char* a_dst = ring + s * T2_STAGE_BYTES;
+                unsigned char* b_dst = a_dst + TC_BM * TC_BK * 2;
+                if (elect_one()) {
                     mbar_expect_tx(full_bar + s, T2_STAGE_BYTES);
                     tma_load_2d(a_dst, &map_a, full_bar + s, kb * TC_BK, row0);
                     tma_load_2d(b_dst, &map_b, full_bar + s, kb * TC_BK, b_row);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, T2_BN);
-            uint32_t g = 0, i = 0;
-            for (int t = blockIdx.x; t < total && !*fail_slot; t += gridDim.x, ++i) {
-                const uint32_t acc = i & 1, use = i >> 1;
-                if (use > 0 && !mbar_wait(acc_empty + acc, (use - 1) & 1)) { *fail_slot = 1; break; }
+        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, T2_BN);
+        uint32_t g = 0, i = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
+            const uint32_t acc = i & 1, use = i >> 1;
+            if (use > 0 && !mbar_wait_warp(acc_empty + acc, (use - 1) & 1)) { *fail_slot = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmem_d = tmem_base + acc * T2_BN;
+            bool ok = true;
+            for (int kb = 0; kb < kblocks; ++kb, ++g) {
+                const uint32_t s = g % T2_STAGES, lap = g / T2_STAGES;
+                if (!mbar_wait_warp(full_bar + s, lap & 1)) { *fail_slot = 1; ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_d = tmem_base + acc * T2_BN;
-                bool ok = true;
-                for (int kb = 0; kb < kblocks; ++kb, ++g) {
-                    const uint32_t s = g % T2_STAGES, lap = g / T2_STAGES;
-                    if (!mbar_wait(full_bar + s, lap & 1)) { *fail_slot = 1; ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = smem_u32(ring + s * T2_STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + TC_BM * TC_BK * 2;
+                const uint32_t a_addr = smem_u32(ring + s * T2_STAGE_BYTES);
+                const uint32_t b_addr = a_addr + TC_BM * TC_BK * 2;
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
                         umma_bf16(tmem_d, umma_desc_sw128(a_addr + k * TC_UMMA_K * 2), umma_desc_sw128(b_addr + k * TC_UMMA_K * 2), idesc,
                                   (kb > 0 || k > 0) ? 1u : 0u);
                     umma_commit(empty_bar + s);
                 }
-                umma_commit(acc_full + acc);  // complete, or abandoned after a timeout: either way release the epilogue
-                if (!ok) break;
+                __syncwarp();
             }
+            if (elect_one()) umma_commit(acc_full + acc);  // complete, or abandoned after a timeout: either way release the epilogue
+            __syncwarp();
+            if (!ok) break;
         }
     } else {
         const int quarter = warp & 3;

@@ -66,6 +66,32 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Roles that feed the tensor core or the TMA run as WHOLE warps: every lane walks the loops and waits, and only the issuing instructions are
+// one lane's, chosen with elect.sync where they are issued.  Their operands are uniform registers; in a loop that only `lane == 0` walks
+// the compiler cannot know that one lane is active, and each tcgen05.mma took 90 - 120 cycles to issue (128 x 256 tiles need 128 per
+// instruction, everything smaller was bound by it).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t mine;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(mine));
+    return mine != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// The warp's index, known to be the same in all its lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 struct TcTile { int row0, row_end, expert, pad; };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
