@@ -13,10 +13,9 @@
 //   attn_final_merge     the head owner waits for the signal, merges the `world` partials in rank order,
 //                        normalizes and stores bf16.
 //
-// The per-row problem is 64 heads x <=2048 gathered keys x 576: far too small and too irregular (every query
-// row has its own key set) to fill a 128-row tcgen05 tile, and it is bound by the gather latency, so the
-// contraction uses warp-level mma.sync m16n8k16 with ldmatrix-fed fragments; the large dense and grouped
-// GEMMs of the model are the tcgen05 kernels.
+// The per-row problem is 64 heads x <=2048 gathered keys x 576, every query row with its own key set.  Decode (a few rows, the
+// chunks are the parallelism) is bound by the gather latency, so its contraction uses warp-level mma.sync m16n8k16 with ldmatrix-fed
+// fragments; many rows of the flagship's head shape run on tcgen05 (sparse_mla_tcgen05.cu).
 //
 // The 2.6 MB selected-row all-reduce of the reference (`glm_tpu/layers/attention/mla.py:484-485`) becomes an
 // exchange of heads x (latent + 2) fp32 per row.  Numerics restate `kernels/sparse_mla/kernel.py:128-183`
@@ -364,6 +363,11 @@ static int launch_rows(const void* q_full, const void* kv_cache, const int* sel_
     return (int)cudaGetLastError();
 }
 
+// sparse_mla_tcgen05.cu
+bool sparse_mla_tc_takes(const void* q_full, const void* kv_cache, const void* o_lat, int H, int L, int rd);
+int launch_sparse_mla_tc(const void* q_full, const void* kv_cache, const int* sel_local, const int* sel_counts, const int* row_lane, int rows,
+                         int layer, int layers, int local_cap, int top_k, float scale, void* o_lat, uint32_t* status, cudaStream_t stream);
+
 // o_lat[rows, H, L] (bf16, normalized) for any number of rows: every selected key of a row lives in this GPU's cache
 // (single GPU, or a replicated cache).  L in {64, 128, 512}; (L + rd) % 16 == 0.
 GLMB_API int glmb_sparse_mla_rows(const void* q_full, const void* kv_cache, const int* sel_local, const int* sel_counts, const int* row_lane,
@@ -371,6 +375,9 @@ GLMB_API int glmb_sparse_mla_rows(const void* q_full, const void* kv_cache, cons
                                   uint32_t* status, void* stream) {
     if (((L + rd) & 15) || rows < 1) return 1;
     cudaStream_t st = (cudaStream_t)stream;
+    // the flagship's head shape at any number of rows (24 rows of 2,048 keys: 170 -> 80 us, 200 of 200: 84 -> 30)
+    if (sparse_mla_tc_takes(q_full, kv_cache, o_lat, H, L, rd))
+        return launch_sparse_mla_tc(q_full, kv_cache, sel_local, sel_counts, row_lane, rows, layer, layers, local_cap, top_k, scale, o_lat, status, st);
 #define ARGS q_full, kv_cache, sel_local, sel_counts, row_lane, rows, H, rd, layer, layers, local_cap, top_k, scale, o_lat, status, st
     if (L == 512) return launch_rows<8, 8>(ARGS);
     if (L == 128) return launch_rows<2, 8>(ARGS);
