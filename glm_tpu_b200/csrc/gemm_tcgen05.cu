@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "peer.cuh"
 #include "tcgen05.cuh"
+#include "gemm_pair_tcgen05.cuh"
 
 #define TC_BM 128
 #define TC_BN 128
@@ -468,6 +469,22 @@ static GemmAllReduce no_allreduce() {
     return ar;
 }
 
+// Columns per tile (256, 192 or 128) of the kernel on pairs of SMs (gemm_pair_tcgen05.cuh), or 0 for the kernels on single SMs: the form whose
+// waves cost least.  A wave of each, relative to 256 x 256 tiles on the 74 pairs ([4096 x 28672], K 4096: 24.6 us a wave): 192 columns
+// 0.79, 128 columns 0.66, 128 x 256 tiles on single SMs 1.17, 128 x 128 tiles on single SMs about 0.9.  Examples, chosen form first: [777 x
+// 6144], K 16384: 192 columns 153 us, 256 columns 199, single 212; [300 x 12288], K 4096: single 39, 192 columns 48, 256 columns 57.
+static int gemm_pair_columns(int rows, int N, int* wave_cost = nullptr) {
+    const int m1 = ceil_div(rows, TC_BM), m2 = ceil_div(rows, 2 * TC_BM), tiles = m1 * ceil_div(N, T2_BN);
+    int best = 0, cost = tiles >= 64 ? 117 * ceil_div(tiles, 148) : 90 * ceil_div(m1 * ceil_div(N, TC_BN), 148);
+    const int columns[3] = {256, 192, 128}, wave[3] = {100, 79, 66};
+    for (int i = 0; i < 3; ++i) {
+        const int c = wave[i] * ceil_div(m2 * ceil_div(N, columns[i]), 74);
+        if (c < cost) { cost = c; best = columns[i]; }
+    }
+    if (wave_cost) *wave_cost = cost;
+    return best;
+}
+
 // a [rows, K] bf16 (lda), b [experts * N, K] bf16 (ldb), c [rows, N] bf16 or fp32 (ldc).  K % 8 == 0; a, b 16-byte
 // aligned with lda, ldb multiples of 8.  tiles / n_tiles: device arrays for grouped mode (max_tiles entries) or NULL.
 GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, int64_t ldb, void* c, int64_t ldc, int rows, int N,
@@ -483,7 +500,9 @@ GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, i
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count < 1) sm_count = 148;
     }
-    // Problems of at least 64 tiles of 128 x 256 run the persistent kernel (measured faster from there on); smaller ones keep 128 x 128 tiles,
+    const int bn = tiles ? 0 : g_gemm_variant >= 32 ? g_gemm_variant : g_gemm_variant == 0 ? gemm_pair_columns(rows, N) : 0;
+    if (bn) return launch_gemm_pair(a, lda, b, nullptr, ldb, c, ldc, rows, N, K, bn, out_f32 ? GP_OUT_F32 : GP_OUT_BF16, 0, status, (cudaStream_t)stream);
+    // On single SMs, problems of at least 64 tiles of 128 x 256 run the persistent kernel (measured faster from there on); smaller ones keep 128 x 128 tiles,
     // which give twice as many CTAs to spread over the SMs.
     const int total2 = m_tiles * ceil_div(N, T2_BN);
     const bool persistent = g_gemm_variant == 2 || (g_gemm_variant == 0 && total2 >= 64);
@@ -509,7 +528,8 @@ GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, i
     return (int)cudaGetLastError();
 }
 
-// 0: choose by problem size; 1: always 128 x 128 tiles, one per CTA; 2: always the persistent 128 x 256 kernel.
+// 0: choose by problem size; 1: always 128 x 128 tiles, one per CTA; 2: always the persistent 128 x 256 kernel; 128, 192, 256: dense problems on
+// pairs of SMs with so many columns per tile.
 GLMB_API void glmb_set_gemm_variant(int variant) { g_gemm_variant = variant; }
 
 // out[rows, N] (bf16, at comm->data[p] + out_offset on EVERY rank p) = sum over ranks of a_r[rows, K_r] . b_r[N, K_r]^T.
@@ -553,4 +573,25 @@ GLMB_API int64_t glmb_gemm_allreduce_part_bytes(int rows, int N, int world) {
     (void)world;  // every rank owns 8 / world blocks of every tile and receives world - 1 (+ its own unused) copies of each
     const int64_t total = (int64_t)ceil_div(rows, TC_BM) * ceil_div(N, T2_BN);
     return total * (int64_t)T2_TILE_FLOATS * 4;
+}
+
+// c[rows, N] (bf16) = f(a . gate^T) * (a . up^T), gate and up [N, K] with the same leading dimension; the products are rounded to bf16
+// before f, as when they pass through memory.  K and N multiples of 8; 16-byte aligned operands with leading dimensions of a multiple of 8.
+GLMB_API int glmb_gemm_bf16_gated(const void* a, int64_t lda, const void* gate, const void* up, int64_t ldb, void* c, int64_t ldc, int rows, int N, int K,
+                                  int kind, uint32_t* status, void* stream) {
+    if (rows < 1 || N < 8 || (N & 7) || K < 8 || (K & 7) || (lda & 7) || (ldb & 7) || (ldc & 7) || (kind != GLU_SILU && kind != GLU_GELU_TANH)) return 1;
+    if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(c)) & 15) return 1;
+    return launch_gemm_pair(a, lda, gate, up, ldb, c, ldc, rows, N, K, 256, GP_OUT_GATED, kind, status, (cudaStream_t)stream);
+}
+
+// Whether that one launch beats the projection of both halves followed by glu_rows: the same tiles of 256 accumulator columns on pairs of SMs
+// against the form gemm_pair_columns picks for 2 N columns (in waves of 24.6 us at K = 4096) and the pass over the [rows, 2 N] result.
+// [4096] x 2 x 14336, K 4096: 697 -> 613 us, [2048] x 2 x 2048, K 6144: 77 -> 72; [300] x 2 x 14336: 93 against 92.  Up to 256 rows a
+// wave is rarely full: [200] x 2 x 12288, K 6144: 80 us in two launches, 87 in one.
+GLMB_API int glmb_gemm_gated_takes(int rows, int N, int K) {
+    if (rows <= 256 || N < 8 || (N & 7) || K < 8 || (K & 7)) return 0;
+    int plain;
+    gemm_pair_columns(rows, 2 * N, &plain);
+    const int gated = 100 * ceil_div(ceil_div(rows, 256) * ceil_div(N, 128), 74);
+    return (gated - plain) * (0.246 * K / 4096) < 2.0 + (double)rows * N * 6 / 4.5e6;
 }

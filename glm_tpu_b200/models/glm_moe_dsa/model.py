@@ -300,6 +300,15 @@ class GlmMoeDsaModel:
         g32, u32 = gate.float(), up.float()  # odd shapes of fixtures only
         return (g32 * torch.sigmoid(g32) * u32).to(torch.bfloat16)
 
+    def _gated(self, x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+        """``bf16(g * sigmoid(g) * u)`` of a prefill chunk's gate and up projections: one launch where that is the faster form."""
+        if (native.gemm_gated_takes(x.shape[0], gate.shape[0], x.shape[1]) and gate.stride() == up.stride()
+                and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, gate, up))):
+            act = torch.empty((x.shape[0], gate.shape[0]), dtype=torch.bfloat16, device=x.device)
+            native.gemm_bf16_gated(x, gate, up, act, native.GLU_SILU, status=self.peer.status_ptr)
+            return act
+        return self._swiglu(self._mm(x, gate), self._mm(x, up))
+
     def _linear_f32(self, x, w, out, decode: bool):
         """``out[:, :N] = x @ w.T`` in fp32."""
         n = w.shape[0]
@@ -537,7 +546,7 @@ class GlmMoeDsaModel:
                     native.skinny_bf16(ws.dense_act[:rows], lw.dense_down, ws.partial, native.SK_OUT_F32)
                     ws.update[:rows] = self._allreduce_rows(ws.partial[:rows]).to(torch.bfloat16)
             else:
-                act = self._swiglu(self._mm(x, lw.dense_gate), self._mm(x, lw.dense_up))
+                act = self._gated(x, lw.dense_gate, lw.dense_up)
                 if self.world == 1:
                     self._mm(act, lw.dense_down, out=ws.update[:rows])
                 else:
@@ -605,7 +614,7 @@ class GlmMoeDsaModel:
                 native.skinny_bf16(ws.act_shared[:rows], lw.shared_down, ws.partial, native.SK_OUT_F32)
             shared_partial = ws.partial
         else:
-            act = self._swiglu(self._mm(x, lw.shared_gate), self._mm(x, lw.shared_up))
+            act = self._gated(x, lw.shared_gate, lw.shared_up)
             library_reduce = not (fused or self.world == 1 or self.emulated_shard)
             # with a library all-reduce ahead the shared partial sums are produced where they will travel from
             both = ws.partial_pair(rows, H) if library_reduce else None

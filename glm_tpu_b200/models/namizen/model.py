@@ -11,7 +11,7 @@ Per layer, five launches in decode:
     chunk_attention   over the lane's ring
     skinny_bf16       [attention | feed-forward] @ [W_o | W_down]: the fp32 update of the residual
 
-In prefill the projections run on the tcgen05 GEMM (gate / up and activation are two launches).  A step whose rows lie in one chunk of a layer
+In prefill the projections run on the tcgen05 GEMM (gate / up and activation are one launch for many rows, two for few).  A step whose rows lie in one chunk of a layer
 attends over the lane's ring itself; one that crosses into another chunk attends over a linear buffer (the chunk so far, copied from the
 ring, then the step's rows), and the rows of the last chunk enter the ring afterwards.
 
@@ -182,7 +182,9 @@ class NamizenModel:
                 native.dual_proj(h1, lw.qkv, proj)
         else:
             self._mm(h1, lw.qkv, proj)
-            if lw.ff_cols:
+            if lw.ff_cols and not self.is_f32 and native.gemm_gated_takes(rows, lw.ff_cols, h2.shape[1]):
+                native.gemm_bf16_gated(h2, lw.gate_up[: lw.ff_cols], lw.gate_up[lw.ff_cols :], act, native.GLU_GELU_TANH, status=self.peer.status_ptr)
+            elif lw.ff_cols:
                 gate_up = ws.gate_up[: rows * 2 * lw.ff_cols].view(rows, 2 * lw.ff_cols)
                 self._mm(h2, lw.gate_up, gate_up)
                 native.glu_rows(gate_up[:, : lw.ff_cols], gate_up[:, lw.ff_cols :], act, native.GLU_GELU_TANH)

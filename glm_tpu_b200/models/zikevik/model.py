@@ -292,6 +292,8 @@ class ZikevikModel:
             act = ws.view("act", rows, F)
             if rows <= native.MAX_ROWS and not self.is_f32:
                 native.skinny_bf16_swiglu(h, t.gate_up[:F], t.gate_up[F:], act)
+            elif not self.is_f32 and native.gemm_gated_takes(rows, F, h.shape[1]):
+                native.gemm_bf16_gated(h, t.gate_up[:F], t.gate_up[F:], act, native.GLU_SILU, status=self.peer.status_ptr)
             else:
                 gate_up = ws.view("gate_up", rows, 2 * F)
                 self._mm(h, t.gate_up, gate_up)

@@ -901,3 +901,23 @@ def gemm_bf16_tc(a, b, out, *, experts=1, tiles=None, n_tiles=None, status=None)
                                      rows, N, K, experts, _p(tiles), _p(n_tiles), max_tiles, out_f32, _p(status), _stream()),
         "gemm_bf16_tcgen05",
     )
+
+
+def gemm_gated_takes(rows: int, N: int, K: int) -> bool:
+    """Whether ``gemm_bf16_gated`` is the faster form of a gated projection (see csrc/gemm_tcgen05.cu)."""
+    lib()
+    return bool(_lib.glmb_gemm_gated_takes(rows, N, K))  # not a launch: past the wrapper that times launches
+
+
+def gemm_bf16_gated(a, gate, up, out, kind, *, status=None):
+    """``out[rows, N] = f(a @ gate.T) * (a @ up.T)`` on the tcgen05 tensor cores, one launch (``kind``: ``GLU_SILU`` or ``GLU_GELU_TANH``).
+
+    ``gate`` and ``up``: bf16 ``[N, K]`` with one leading dimension; ``out``: bf16 rows, possibly a column range of wider ones."""
+    rows, K = a.shape
+    if up.stride(0) != gate.stride(0) or tuple(up.shape) != tuple(gate.shape):
+        raise ValueError("gate and up have the same shape and strides")
+    _check(
+        lib().glmb_gemm_bf16_gated(_p(a), C.c_int64(a.stride(0)), _p(gate), _p(up), C.c_int64(gate.stride(0)), _p(out), C.c_int64(out.stride(0)),
+                                   rows, gate.shape[0], K, int(kind), _p(status), _stream()),
+        "gemm_bf16_gated",
+    )
