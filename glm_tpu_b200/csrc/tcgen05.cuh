@@ -168,21 +168,3 @@ static inline int make_map(CUtensorMap* map, const void* base, uint64_t rows, ui
         return r == CUDA_SUCCESS ? 0 : 2;
     });
 }
-
-
-// [rows, K] bytes row-major (leading dimension ld bytes), box `box_rows` rows x 64 bytes, no swizzle: FP8 weight tiles
-// that CUDA threads (not the tensor core) read back from shared memory.
-static inline int make_map_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint64_t ld, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_tiled();
-    if (!fn) return 1;
-    return cached_map(map, TensorMapKey{1, base, rows, K, ld, box_rows}, [&](CUtensorMap* out) {
-        const cuuint64_t dims[2] = {K, rows};
-        const cuuint64_t strides[1] = {ld};
-        const cuuint32_t box[2] = {64, box_rows};
-        const cuuint32_t elem[2] = {1, 1};
-        CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        return r == CUDA_SUCCESS ? 0 : 2;
-    });
-}
