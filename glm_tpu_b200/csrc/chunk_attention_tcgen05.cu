@@ -42,14 +42,6 @@ __device__ __forceinline__ void fa_tmem_st16(uint32_t taddr, const uint32_t (&r)
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
         "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
-// D[tmem] (+)= A[tmem] . B[shared]
-__device__ __forceinline__ void fa_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
 // MN-major operand, 128-byte swizzle: 64 columns (128 bytes) per K row, 8 K rows per 1024-byte group, 64-column boxes FA_BOX apart
 __device__ __forceinline__ uint64_t fa_desc_mn(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(FA_BOX >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
@@ -146,7 +138,7 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         for (int piece = 0; piece < 2; ++piece)
 #pragma unroll
                             for (int k = 0; k < FA_TILE / 16; ++k)
-                                fa_mma_ts(tmem + 256 + t * 128, tmem + t * 128 + piece * 64 + k * 8, fa_desc_mn(v_addr + k * 2048), idesc_o,
+                                umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + piece * 64 + k * 8, fa_desc_mn(v_addr + k * 2048), idesc_o,
                                           (done[t] > 0 || piece > 0 || k > 0) ? 1u : 0u);
                         if (j + 1 == range[t].end) umma_commit(o_full + t);
                     }

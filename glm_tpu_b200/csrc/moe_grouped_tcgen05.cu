@@ -8,20 +8,22 @@
 // expert (gate/up: 128 gate rows and the 128 up rows of the same outputs) x up to 128 routes; one CTA per SM walks the tiles, all
 // column blocks of a route tile after each other, so that neighbouring CTAs share the activations in L2.  Per 128-wide k step:
 //
-//   warps 6-21   decode, a team of eight warps per matrix: 64 codes per thread, straight from global memory (a piece is asked for again,
-//                for two steps later, as soon as it has been decoded), block scale in fp32, rounded to bf16 (the weight-decode
-//                contract), into two 64-column boxes in the 128-byte-swizzled K-major layout of the tensor core; a proxy fence
-//                publishes them.  A team has two such stages, so that it decodes one while the tensor core reads the other
-//   warp 0       TMA: the activations of the tile's routes (32-row boxes, as many as there are routes)
-//   warp 1       issues tcgen05.mma (two matrices of M 128, N 16 .. 128) into one of two sets of TMEM accumulators
+//   warp 0       TMA: the FP8 rows of both matrices (128-byte swizzle, four steps in flight), and the activations of the tile's routes
+//                (32-row boxes, as many as there are routes)
+//   warps 6-21   decode: a thread owns half the columns of a weight row, 64 codes; block scale in fp32, rounded to bf16 (the
+//                weight-decode contract), into TENSOR MEMORY, which the tensor core reads as its A operand: decoded weights that went
+//                through shared memory (64 KB written and 64 KB read a step) were what bound this kernel.  Two stages per matrix
+//   warp 1       issues tcgen05.mma (two matrices of M 128, N 16 .. 128)
 //   warps 2-5    epilogue of the tile before, while the next one is decoded and multiplied: a thread owns a weight row (TMEM lane)
 //                  gate/up mode  act = bf16( silu(bf16 gate) * bf16 up ), stored in sorted order
 //                  down mode     dw[route] = bf16( bf16(acc) * bf16(route weight) ), scattered to the route's slot
 //
-// What bounds it: shared-memory traffic (decoded weights in and out to the tensor core, activations) and the decoding, at 3.3 TB/s of weights
-// whatever the number of routes; prefetching whole stretches of a row into the L2 changes nothing.  Measured on a B200, [256 experts, 2 x 2048 x
-// 6144] and back, against routes as the M in tiles of 128 and weights through shared memory twice: 2,048 rows 2,377 + 1,302 -> 1,891 + 1,034 us,
-// 777 rows 1,931 + 1,065 -> 1,680 + 856.
+// TMEM: 256 columns of accumulators (two tiles of up to 64 routes, or one of more), 256 of decoded weights.
+//
+// What bounds it: the FP8 bytes, which cross HBM once (5.2 - 5.7 TB/s up to 777 rows), and with many routes the epilogue of tiles of more than
+// 64 routes, which have one accumulator.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 1,061 + 554 us
+// (routes as the M in tiles of 128: 1,931 + 1,065; decoded weights through shared memory: 1,680 + 856); 2,048 rows 1,593 + 1,007 (2,377 +
+// 1,302; 1,891 + 1,034).
 // Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores and
 // still frees its TMEM.
 //
@@ -35,18 +37,17 @@
 #define MG_BK 128
 #define MG_BOX 16384   // bytes of 128 rows x 64 bf16 columns
 #define MG_STAGES 3    // activations: two boxes each
-#define MG_WSTAGES 4   // decoded weights: two of each matrix, two boxes each
-#define MG_TEAM_WARPS 8
-#define MG_THREADS (6 * 32 + 2 * 32 * MG_TEAM_WARPS)
-#define MG_SMEM_BYTES ((MG_STAGES * 2 + MG_WSTAGES * 2) * MG_BOX + 1024)
+#define MG_RAW 4       // FP8 weights: 128 rows x 128 bytes of each matrix
+#define MG_CONV_WARPS 16
+#define MG_THREADS (6 * 32 + 32 * MG_CONV_WARPS)
+#define MG_SMEM_BYTES ((MG_STAGES * 2 + MG_RAW * 2) * MG_BOX + 1024)
+#define MG_A_COL 256   // TMEM column of the decoded weights: stage j of matrix m at 64 (2 m + j) from here
 
 struct MoeGroupedArgs {
     const TcTile* tiles;      // [max_tiles] 128-route tiles of the expert-sorted route list (row0, the expert's row_end, local expert)
     const int* n_tiles;       // [1] on the device
-    const uint8_t* w0;        // [experts, N, K] FP8: gate, or down
-    const uint8_t* w1;        // up (gate/up mode), or down again
-    const float* scale0;      // block scales of w0 [experts, ceil(N/128), ceil(K/128)]
-    const float* scale1;      // ... of w1
+    const float* scale0;      // block scales of the first weight [experts, ceil(N/128), ceil(K/128)]
+    const float* scale1;      // ... of the second (gate/up mode: up; down mode: the same table)
     const int* perm;          // [sorted routes] -> route id (row * top_k + slot), -1 for none   (down mode)
     const float* route_weight;  // [routes] fp32                                                  (down mode)
     bf16* out;                // gate/up: act_sorted [sorted routes, N];  down: dw [routes, N]
@@ -55,14 +56,43 @@ struct MoeGroupedArgs {
     uint32_t* status;
 };
 
-__global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, MoeGroupedArgs a) {
+// Which accumulator columns an item takes: a tile of up to 64 routes one of the two halves, in turn, a larger one both.  Every role that meets the
+// accumulators walks the same items and keeps the same counts, which are the phases of the halves' barriers.
+struct MgHalves {
+    uint32_t uses[2] = {0, 0};
+    bool wide = false;
+    int half = 0;
+    __device__ __forceinline__ void next(int routes) {
+        wide = routes > 64;
+        half = uses[0] <= uses[1] ? 0 : 1;
+    }
+    __device__ __forceinline__ bool takes(int h) const { return wide || h == half; }
+    __device__ __forceinline__ uint32_t column(int matrix) const { return wide ? matrix * 128 : half * 128 + matrix * 64; }
+    __device__ __forceinline__ void done() {
+        if (takes(0)) ++uses[0];
+        if (takes(1)) ++uses[1];
+    }
+};
+
+__device__ __forceinline__ void mg_tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
+        "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+
+__global__ void __launch_bounds__(MG_THREADS, 1)
+moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                        MoeGroupedArgs a) {
     GLMB_PDL_PROLOGUE();
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t x_full[MG_STAGES], x_empty[MG_STAGES], w_full[MG_WSTAGES], w_empty[MG_WSTAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t x_full[MG_STAGES], x_empty[MG_STAGES], raw_full[MG_RAW], raw_empty[MG_RAW], w_full[4], w_empty[4], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t fail;
     unsigned char* x_s = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* w_s = x_s + MG_STAGES * 2 * MG_BOX;
+    unsigned char* raw_s = x_s + MG_STAGES * 2 * MG_BOX;
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int cols = a.mode == 0 ? 128 : 256;  // output columns of a tile
     const int blocks = (a.N + cols - 1) / cols, steps = (a.K + MG_BK - 1) / MG_BK;
@@ -70,7 +100,8 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MG_STAGES; ++s) { mbar_init(x_full + s, 1); mbar_init(x_empty + s, 1); }
-        for (int j = 0; j < MG_WSTAGES; ++j) { mbar_init(w_full + j, MG_TEAM_WARPS); mbar_init(w_empty + j, 1); }
+        for (int s = 0; s < MG_RAW; ++s) { mbar_init(raw_full + s, 1); mbar_init(raw_empty + s, MG_CONV_WARPS); }
+        for (int j = 0; j < 4; ++j) { mbar_init(w_full + j, MG_CONV_WARPS / 2); mbar_init(w_empty + j, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4); }
         fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -82,7 +113,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;  // accumulator set i at 256 i: matrix 0, then matrix 1, a column per route
+    const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
         uint32_t g = 0;  // steps so far, over the items of this CTA
@@ -90,8 +121,16 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             const TcTile t = a.tiles[it / blocks];
             const int boxes = (min(t.row_end - t.row0, MG_ROUTES) + 31) >> 5;
+            const int w_row = t.expert * a.N + (it % blocks) * cols, w_row1 = a.mode == 0 ? w_row : w_row + 128;  // rows past N are never stored
             for (int kb = 0; kb < steps; ++kb, ++g) {
-                const uint32_t s = g % MG_STAGES, lap = g / MG_STAGES;
+                const uint32_t s = g % MG_STAGES, lap = g / MG_STAGES, q = g % MG_RAW, raw_lap = g / MG_RAW;
+                if (raw_lap > 0 && !mbar_wait_warp(raw_empty + q, (raw_lap - 1) & 1)) { fail = 1; ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(raw_full + q, 2 * MG_BOX);
+                    tma_load_2d(raw_s + q * 2 * MG_BOX, &map_w0, raw_full + q, kb * MG_BK, w_row);
+                    tma_load_2d(raw_s + (q * 2 + 1) * MG_BOX, &map_w1, raw_full + q, kb * MG_BK, w_row1);
+                }
+                __syncwarp();
                 if (lap > 0 && !mbar_wait_warp(x_empty + s, (lap - 1) & 1)) { fail = 1; ok = false; break; }
                 if (elect_one()) {
                     mbar_expect_tx(x_full + s, boxes * 2 * 4096);
@@ -103,134 +142,117 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
             }
         }
     } else if (warp == 1) {
-        uint32_t g = 0, i = 0;
-        for (int it = blockIdx.x; it < items; it += gridDim.x, ++i) {
+        uint32_t g = 0;
+        MgHalves at;
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const TcTile t = a.tiles[it / blocks];
-            const uint32_t acc = i & 1, use = i >> 1;
             const int routes = min(max((t.row_end - t.row0 + 15) & ~15, 16), MG_ROUTES);
             const uint32_t idesc = umma_idesc_bf16(128, routes);
-            if (use > 0 && !mbar_wait_warp(acc_empty + acc, (use - 1) & 1)) { fail = 1; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            at.next(routes);
             bool ok = true;
-            for (int kb = 0; kb < steps; ++kb, ++g) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (ok && at.takes(h) && at.uses[h] > 0) ok = mbar_wait_warp(acc_empty + h, (at.uses[h] - 1) & 1);
+            if (!ok) { fail = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int kb = 0; kb < steps && ok; ++kb, ++g) {
                 const uint32_t s = g % MG_STAGES;
-                if (!mbar_wait_warp(x_full + s, (g / MG_STAGES) & 1)) { fail = 1; ok = false; break; }
+                ok = mbar_wait_warp(x_full + s, (g / MG_STAGES) & 1);
                 const uint32_t x_addr = smem_u32(x_s + s * 2 * MG_BOX);
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
                     const uint32_t j = m * 2 + (g & 1);
-                    if (ok && !mbar_wait_warp(w_full + j, (g >> 1) & 1)) { fail = 1; ok = false; }
+                    if (ok) ok = mbar_wait_warp(w_full + j, (g >> 1) & 1);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t w_addr = smem_u32(w_s + j * 2 * MG_BOX);
                     if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < MG_BK / 16; ++k) {
-                            const uint32_t at = (k >> 2) * MG_BOX + (k & 3) * 32;
-                            umma_bf16(tmem + acc * 256 + m * 128, umma_desc_sw128(w_addr + at), umma_desc_sw128(x_addr + at), idesc,
-                                      (kb > 0 || k > 0) ? 1u : 0u);
-                        }
+                        for (int k = 0; k < MG_BK / 16; ++k)
+                            umma_bf16_ts(tmem + at.column(m), tmem + MG_A_COL + j * 64 + k * 8, umma_desc_sw128(x_addr + (k >> 2) * MG_BOX + (k & 3) * 32), idesc,
+                                         (kb > 0 || k > 0) ? 1u : 0u);
                         umma_commit(w_empty + j);
                         if (m == 1) umma_commit(x_empty + s);
                     }
                     __syncwarp();
                 }
-                if (!ok) break;
             }
-            if (elect_one()) umma_commit(acc_full + acc);  // complete, or abandoned after a timeout: either way release the epilogue
+            if (!ok) fail = 1;
+            if (elect_one()) {  // complete, or abandoned after a timeout: either way release the epilogue
+                if (at.takes(0)) umma_commit(acc_full);
+                if (at.takes(1)) umma_commit(acc_full + 1);
+            }
             __syncwarp();
             if (!ok) break;
+            at.done();
         }
     } else if (warp >= 6) {
-        // ---- decode: team = matrix; thread (row % 32, piece of 16 codes) of 128 rows ----------------------------------------------
-        const int team = (warp - 6) / MG_TEAM_WARPS, dt = threadIdx.x - 192 - team * MG_TEAM_WARPS * 32, row = dt >> 3, c = dt & 7;
+        // ---- decode: thread = weight row = TMEM lane; four sets of four warps: (matrix, half of the step's columns) -------------------
+        const int set = (warp - 6) >> 2, m = set >> 1, half = set & 1, quarter = warp & 3, row = quarter * 32 + lane;
         const int n_srows = (a.N + 127) >> 7, n_scols = (a.K + 127) >> 7;
-        const int mine = (int)blockIdx.x < items ? (items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-        const int total = mine * steps, second = a.mode == 1 && team ? 128 : 0;  // where the team's columns begin in the tile
-        const uint8_t* const table = team ? a.w1 : a.w0;
-        const float* const scales = team ? a.scale1 : a.scale0;
-        int l_it = blockIdx.x, l_kb = 0, l_step = 0, below = 0;  // the step whose codes are asked for next; rows from this thread's first one to N
-        const uint8_t* base = nullptr;
-        const float* sc = nullptr;
-        auto aim = [&]() {
-            if (l_step >= total) return;
-            const int expert = a.tiles[l_it / blocks].expert, n0 = (l_it % blocks) * cols + second;
-            below = a.N - n0 - row;
-            base = table + ((int64_t)expert * a.N + n0 + row) * a.K + c * 16;
-            sc = scales + ((int64_t)expert * n_srows + min(n0 >> 7, n_srows - 1)) * n_scols;
-        };
-        uint4 w[2][4];
-        float s[2] = {0.f, 0.f};
-        auto load = [&](uint4& to, int i) {
-            const int k = l_kb * MG_BK;
-            const bool in = l_step < total && k + c * 16 < a.K && i * 32 < below;
-            to = in ? ld_stream16(base + (int64_t)(i * 32) * a.K + k) : make_uint4(0, 0, 0, 0);
-        };
-        auto onward = [&]() {
-            ++l_step;
-            if (++l_kb == steps) { l_kb = 0; l_it += gridDim.x; aim(); }
-        };
-        aim();
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            if (l_step < total) s[p] = __ldg(sc + l_kb);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) load(w[p][i], i);
-            onward();
-        }
-        // eight lanes hold a row's 128 columns: a quarter warp's first stores take the even chunks of the lower box and the odd ones
-        // of the upper, so that they meet eight different groups of banks
-        const int odd = c >> 2, chunk = (c & 3) * 2;
-        unsigned char* line = w_s + team * 4 * MG_BOX + odd * MG_BOX + (row >> 3) * 1024 + (row & 7) * 128;
-        unsigned char *at0 = line + (((chunk + odd) ^ (row & 7)) << 4), *at1 = line + (((chunk + 1 - odd) ^ (row & 7)) << 4);
+        const float* const scales = m ? a.scale1 : a.scale0;
+        const uint32_t a_addr = tmem + ((uint32_t)(quarter * 32) << 16) + MG_A_COL + m * 128 + half * 32;
+        const unsigned char* const line = raw_s + m * MG_BOX + row * 128;
+        uint32_t g = 0;
         bool ok = true;
-        for (int step = 0; step < total && ok; step += 2) {
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            const int n0 = (it % blocks) * cols + (a.mode == 1 ? m * 128 : 0);
+            const float* sc = scales + ((int64_t)a.tiles[it / blocks].expert * n_srows + min(n0 >> 7, n_srows - 1)) * n_scols;
+            float next = __ldg(sc);
+            for (int kb = 0; kb < steps; ++kb, ++g) {
+                const uint32_t q = g % MG_RAW, j = g & 1, lap = g >> 1;
+                const float scale = next;
+                next = __ldg(sc + min(kb + 1, n_scols - 1));
+                if (!mbar_wait_warp(raw_full + q, (g / MG_RAW) & 1)) { fail = 1; ok = false; break; }
+                uint4 w[4];
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                if (step + p >= total) break;
-                const uint32_t j = team * 2 + p, lap = step >> 1;
-                if (lap > 0 && !mbar_wait_warp(w_empty + j, (lap - 1) & 1)) { fail = 1; ok = false; break; }
-                const float scale = s[p];
-                if (l_step < total) s[p] = __ldg(sc + l_kb);
+                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const uint4*>(line + q * 2 * MG_BOX + (((half * 4 + i) ^ (row & 7)) << 4));
+                uint32_t v[32];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint4 v = w[p][i];
-                    const uint4 lo = make_uint4(dec2(v.x, scale), dec2(v.x >> 16, scale), dec2(v.y, scale), dec2(v.y >> 16, scale));
-                    const uint4 hi = make_uint4(dec2(v.z, scale), dec2(v.z >> 16, scale), dec2(v.w, scale), dec2(v.w >> 16, scale));
-                    load(w[p][i], i);
-                    const int to = p * 2 * MG_BOX + i * 32 * 128;
-                    *reinterpret_cast<uint4*>(at0 + to) = odd ? hi : lo;
-                    *reinterpret_cast<uint4*>(at1 + to) = odd ? lo : hi;
+                    const uint32_t c[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        v[i * 8 + 2 * p] = dec2(c[p], scale);
+                        v[i * 8 + 2 * p + 1] = dec2(c[p] >> 16, scale);
+                    }
                 }
-                onward();
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the tensor core
                 __syncwarp();
-                if (lane == 0) mbar_arrive(w_full + j);
+                if (lane == 0) mbar_arrive(raw_empty + q);
+                if (lap > 0 && !mbar_wait_warp(w_empty + m * 2 + j, (lap - 1) & 1)) { fail = 1; ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                mg_tmem_st32(a_addr + j * 64, v);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(w_full + m * 2 + j);
             }
         }
     } else {
         // ---- epilogue: thread = weight row = TMEM lane; neighbouring lanes swap, so that each stores two columns of one route -----------
         const int quarter = warp & 3;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        uint32_t i = 0;
-        for (int it = blockIdx.x; it < items; it += gridDim.x, ++i) {
+        MgHalves at;
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const TcTile t = a.tiles[it / blocks];
-            const uint32_t acc = i & 1;
-            const bool done = mbar_wait_warp(acc_full + acc, (i >> 1) & 1);
+            const int routes = min(t.row_end - t.row0, MG_ROUTES), n0 = (it % blocks) * cols + quarter * 32 + (lane & ~1);
+            at.next(min(max((routes + 15) & ~15, 16), MG_ROUTES));
+            bool done = true;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (done && at.takes(h)) done = mbar_wait_warp(acc_full + h, at.uses[h] & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!done || __any_sync(0xffffffffu, fail)) {
                 fail = 1;
                 if (lane == 0) raise_status(a.status, GLMB_STATUS_WAIT_TIMEOUT);
                 break;
             }
-            const int routes = min(t.row_end - t.row0, MG_ROUTES), n0 = (it % blocks) * cols + quarter * 32 + (lane & ~1);
-            const uint32_t d = tmem + acc * 256 + lanes;
+            const uint32_t d0 = tmem + lanes + at.column(0), d1 = tmem + lanes + at.column(1);
 #pragma unroll 1
             for (int r0 = 0; r0 < routes; r0 += 16) {
                 if (a.mode == 0) {
                     uint32_t g[16], u[16];
-                    tmem_ld16(d + r0, g);
-                    tmem_ld16(d + 128 + r0, u);
+                    tmem_ld16(d0 + r0, g);
+                    tmem_ld16(d1 + r0, u);
 #pragma unroll
                     for (int e = 0; e < 16; e += 2) {
                         float v[2];
@@ -252,7 +274,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
                         uint32_t x[16];
-                        tmem_ld16(d + m * 128 + r0, x);
+                        tmem_ld16((m ? d1 : d0) + r0, x);
 #pragma unroll
                         for (int e = 0; e < 16; e += 2) {
                             const float v0 = bf16_round(__uint_as_float(x[e])) * __shfl_sync(0xffffffffu, weight, e);
@@ -267,7 +289,11 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_grouped_fp8w_kernel(const _
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + acc);
+            if (lane == 0) {
+                if (at.takes(0)) mbar_arrive(acc_empty);
+                if (at.takes(1)) mbar_arrive(acc_empty + 1);
+            }
+            at.done();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -303,8 +329,10 @@ GLMB_API int glmb_moe_grouped_fp8w(const void* a_sorted, int sorted_rows, const 
     if (mode == 1 && (!perm || !route_weight)) return 1;
     if ((reinterpret_cast<uintptr_t>(a_sorted) & 15) || (reinterpret_cast<uintptr_t>(w0) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return 1;
     if (mode == 0 && (!w1 || !s1 || (reinterpret_cast<uintptr_t>(w1) & 15))) return 1;
-    CUtensorMap map_a;
+    CUtensorMap map_a, map_w0, map_w1;
     if (make_map(&map_a, a_sorted, (uint64_t)sorted_rows, (uint64_t)K, (uint64_t)K, 32)) return 3;
+    if (make_map_u8(&map_w0, w0, (uint64_t)experts * N, (uint64_t)K, (uint64_t)K, 128)) return 3;
+    if (make_map_u8(&map_w1, mode == 0 ? w1 : w0, (uint64_t)experts * N, (uint64_t)K, (uint64_t)K, 128)) return 3;
     static DeviceOnce attr_set;
     const int attr_set_dev = attr_set.pending();
     if (attr_set_dev != DeviceOnce::SET) {
@@ -315,8 +343,6 @@ GLMB_API int glmb_moe_grouped_fp8w(const void* a_sorted, int sorted_rows, const 
     MoeGroupedArgs args;
     args.tiles = (const TcTile*)tiles;
     args.n_tiles = n_tiles;
-    args.w0 = (const uint8_t*)w0;
-    args.w1 = (const uint8_t*)(mode == 0 ? w1 : w0);
     args.scale0 = s0;
     args.scale1 = mode == 0 ? s1 : s0;
     args.perm = perm;
@@ -325,7 +351,7 @@ GLMB_API int glmb_moe_grouped_fp8w(const void* a_sorted, int sorted_rows, const 
     args.N = N; args.K = K; args.mode = mode; args.max_tiles = max_tiles;
     args.status = status;
     const int64_t most = (int64_t)(mode == 0 ? ceil_div(N, 128) : ceil_div(N, 256)) * max_tiles;
-    GLMB_LAUNCH(moe_grouped_fp8w_kernel, (int)(most < 148 ? most : 148), MG_THREADS, MG_SMEM_BYTES, (cudaStream_t)stream, map_a, args);
+    GLMB_LAUNCH(moe_grouped_fp8w_kernel, (int)(most < 148 ? most : 148), MG_THREADS, MG_SMEM_BYTES, (cudaStream_t)stream, map_a, map_w0, map_w1, args);
     return (int)cudaGetLastError();
 }
 

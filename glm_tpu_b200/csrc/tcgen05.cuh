@@ -92,6 +92,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// D[tmem] (+)= A[tmem] . B[shared]
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 struct TcTile { int row0, row_end, expert, pad; };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -163,6 +172,23 @@ static inline int make_map(CUtensorMap* map, const void* base, uint64_t rows, ui
         const cuuint32_t box[2] = {64, box_rows};
         const cuuint32_t elem[2] = {1, 1};
         CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        return r == CUDA_SUCCESS ? 0 : 2;
+    });
+}
+
+// [rows, K] bytes row-major (leading dimension ld bytes), box `box_rows` rows x 128 bytes, 128-byte swizzle: FP8 weight tiles
+// that CUDA threads read back from shared memory.
+static inline int make_map_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint64_t ld, uint32_t box_rows) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return 1;
+    return cached_map(map, TensorMapKey{1, base, rows, K, ld, box_rows}, [&](CUtensorMap* out) {
+        const cuuint64_t dims[2] = {K, rows};
+        const cuuint64_t strides[1] = {ld};
+        const cuuint32_t box[2] = {128, box_rows};
+        const cuuint32_t elem[2] = {1, 1};
+        CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         return r == CUDA_SUCCESS ? 0 : 2;
