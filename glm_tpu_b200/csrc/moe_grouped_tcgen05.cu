@@ -23,7 +23,7 @@
 // What bounds it: the FP8 bytes, which cross HBM once (5.2 - 5.7 TB/s up to 777 rows), and with many routes the epilogue of tiles of more than
 // 64 routes, which have one accumulator.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 1,061 + 554 us
 // (routes as the M in tiles of 128: 1,931 + 1,065; decoded weights through shared memory: 1,680 + 856); 2,048 rows 1,593 + 1,007 (2,377 +
-// 1,302; 1,891 + 1,034).
+// 1,302; 1,891 + 1,034), and 1,413 + 799 since the epilogue has no division and no per-column loads of the route list.
 // Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores and
 // still frees its TMEM.
 //
@@ -236,6 +236,14 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             const TcTile t = a.tiles[it / blocks];
             const int routes = min(t.row_end - t.row0, MG_ROUTES), n0 = (it % blocks) * cols + quarter * 32 + (lane & ~1);
             at.next(min(max((routes + 15) & ~15, 16), MG_ROUTES));
+            int route[4];  // of columns lane, lane + 32, ..: asked for while the products are still under way
+            float weight[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = i * 32 + lane;
+                route[i] = a.mode == 1 && r < routes ? a.perm[t.row0 + r] : -1;
+                weight[i] = route[i] >= 0 ? bf16_round(a.route_weight[route[i]]) : 0.f;
+            }
             bool done = true;
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -259,7 +267,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             const float gv = bf16_round(__uint_as_float(g[e + q])), uv = bf16_round(__uint_as_float(u[e + q]));
-                            v[q] = gv * sigmoidf_precise(gv) * uv;
+                            v[q] = gv * __fdividef(1.f, 1.f + expf(-gv)) * uv;  // no branch: an IEEE division would serialise the elements
                         }
                         const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[0] : v[1], 1);
                         const int r = r0 + e + (lane & 1);
@@ -267,22 +275,23 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                             *reinterpret_cast<uint32_t*>(a.out + (int64_t)(t.row0 + r) * a.N + n0) = (lane & 1) ? pack_bf16(got, v[1]) : pack_bf16(v[0], got);
                     }
                 } else {
-                    int route = -1;  // of column r0 + lane
-                    float weight = 0.f;
-                    if (lane < 16 && r0 + lane < routes) route = a.perm[t.row0 + r0 + lane];
-                    if (route >= 0) weight = bf16_round(a.route_weight[route]);
+                    const int q = r0 >> 5, at32 = r0 & 31;
+                    const int routes32 = q < 2 ? (q ? route[1] : route[0]) : (q & 1 ? route[3] : route[2]);
+                    const float weights32 = q < 2 ? (q ? weight[1] : weight[0]) : (q & 1 ? weight[3] : weight[2]);
+                    uint32_t x[2][16];
+                    tmem_ld16(d0 + r0, x[0]);
+                    tmem_ld16(d1 + r0, x[1]);
 #pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        uint32_t x[16];
-                        tmem_ld16((m ? d1 : d0) + r0, x);
+                    for (int e = 0; e < 16; e += 2) {
+                        const int to = __shfl_sync(0xffffffffu, routes32, at32 + e + (lane & 1));
+                        const float w0 = __shfl_sync(0xffffffffu, weights32, at32 + e), w1 = __shfl_sync(0xffffffffu, weights32, at32 + e + 1);
+                        bf16* dst = a.out + (int64_t)to * a.N + n0;
 #pragma unroll
-                        for (int e = 0; e < 16; e += 2) {
-                            const float v0 = bf16_round(__uint_as_float(x[e])) * __shfl_sync(0xffffffffu, weight, e);
-                            const float v1 = bf16_round(__uint_as_float(x[e + 1])) * __shfl_sync(0xffffffffu, weight, e + 1);
+                        for (int m = 0; m < 2; ++m) {
+                            const float v0 = bf16_round(__uint_as_float(x[m][e])) * w0, v1 = bf16_round(__uint_as_float(x[m][e + 1])) * w1;
                             const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v0 : v1, 1);
-                            const int to = __shfl_sync(0xffffffffu, route, e + (lane & 1));
                             if (to >= 0 && n0 + m * 128 < a.N)
-                                *reinterpret_cast<uint32_t*>(a.out + (int64_t)to * a.N + n0 + m * 128) = (lane & 1) ? pack_bf16(got, v1) : pack_bf16(v0, got);
+                                *reinterpret_cast<uint32_t*>(dst + m * 128) = (lane & 1) ? pack_bf16(got, v1) : pack_bf16(v0, got);
                         }
                     }
                 }
