@@ -195,10 +195,21 @@ __device__ __forceinline__ void t2_tile(int t, int m_tiles, int n_blocks, int& m
     n = (t % group) / gm;
 }
 
+// Problems side by side (per-head products): problem h reads A from column h a_cols, B from row h b_rows + b_row0 and writes C from column
+// h c_cols.  MN: B lies as [K, N] (its rows are the k's).
+struct GemmBatch {
+    int count = 1, a_cols = 0, b_rows = 0, b_row0 = 0, c_cols = 0;
+};
+// MN-major operand of 64 k rows, 128-byte swizzle: 64 columns per k row, 8 k rows per 1024-byte group, 64-column boxes 8,192 bytes apart
+__device__ __forceinline__ uint64_t t2_desc_mn(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+template <bool MN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                     void* __restrict__ c, int64_t ldc, int rows, int N, int K, const TcTile* __restrict__ tiles,
-                                    const int* __restrict__ n_tiles, int max_tiles, int out_f32, uint32_t* status, GemmAllReduce ar) {
+                                    const int* __restrict__ n_tiles, int max_tiles, int out_f32, uint32_t* status, GemmAllReduce ar, GemmBatch batch) {
     GLMB_PDL_PROLOGUE();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -215,7 +226,7 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     const uint32_t ar_epoch = ar.enabled ? ar.comm.seq[GLMB_SEQ_GEMM] + 1 : 0;
     const int m_tiles = tiles ? min(max(*n_tiles, 0), max_tiles) : (rows + TC_BM - 1) / TC_BM;
     const int n_blocks = (N + T2_BN - 1) / T2_BN;
-    const int total = m_tiles * n_blocks;
+    const int per_problem = m_tiles * n_blocks, total = per_problem * batch.count;
     const int kblocks = (K + TC_BK - 1) / TC_BK;
 
     if (threadIdx.x == 0) {
@@ -238,9 +249,11 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int m, n;
-            t2_tile(t, m_tiles, n_blocks, m, n);
+            const int head = t / per_problem;
+            t2_tile(t % per_problem, m_tiles, n_blocks, m, n);
             const int row0 = tiles ? tiles[m].row0 : m * TC_BM;
-            const int b_row = (tiles ? tiles[m].expert : 0) * N + n * T2_BN;
+            const int a_col = head * batch.a_cols;
+            const int b_row = MN ? head * batch.b_rows + batch.b_row0 : (tiles ? tiles[m].expert : 0) * N + head * batch.b_rows + batch.b_row0 + n * T2_BN;
             for (int kb = 0; kb < kblocks; ++kb, ++g) {
                 const uint32_t s = g % T2_STAGES, lap = g / T2_STAGES;
                 if (lap > 0 && !mbar_wait_warp(empty_bar + s, (lap - 1) & 1)) { *fail_slot = 1; ok = false; break; }
@@ -248,14 +261,17 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
                 unsigned char* b_dst = a_dst + TC_BM * TC_BK * 2;
                 if (elect_one()) {
                     mbar_expect_tx(full_bar + s, T2_STAGE_BYTES);
-                    tma_load_2d(a_dst, &map_a, full_bar + s, kb * TC_BK, row0);
-                    tma_load_2d(b_dst, &map_b, full_bar + s, kb * TC_BK, b_row);
+                    tma_load_2d(a_dst, &map_a, full_bar + s, a_col + kb * TC_BK, row0);
+                    if (MN)
+                        for (int b = 0; b < T2_BN / 64; ++b) tma_load_2d(b_dst + b * 8192, &map_b, full_bar + s, n * T2_BN + b * 64, b_row + kb * TC_BK);
+                    else
+                        tma_load_2d(b_dst, &map_b, full_bar + s, kb * TC_BK, b_row);
                 }
                 __syncwarp();
             }
         }
     } else if (warp == 1) {
-        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, T2_BN);
+        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, T2_BN) | (MN ? 1u << 16 : 0u);  // bit 16: B is MN-major
         uint32_t g = 0, i = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
             const uint32_t acc = i & 1, use = i >> 1;
@@ -272,8 +288,8 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
-                        umma_bf16(tmem_d, umma_desc_sw128(a_addr + k * TC_UMMA_K * 2), umma_desc_sw128(b_addr + k * TC_UMMA_K * 2), idesc,
-                                  (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_bf16(tmem_d, umma_desc_sw128(a_addr + k * TC_UMMA_K * 2),
+                                  MN ? t2_desc_mn(b_addr + k * 2048) : umma_desc_sw128(b_addr + k * TC_UMMA_K * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     umma_commit(empty_bar + s);
                 }
                 __syncwarp();
@@ -294,7 +310,8 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
                 break;
             }
             int m, n;
-            t2_tile(t, m_tiles, n_blocks, m, n);
+            const int head = t / per_problem;
+            t2_tile(t % per_problem, m_tiles, n_blocks, m, n);
             const int row0 = tiles ? tiles[m].row0 : m * TC_BM;
             const int row_end = tiles ? tiles[m].row_end : rows;
             const int row = row0 + quarter * 32 + lane;
@@ -408,14 +425,14 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
                 if (row < row_end && col < N) {
 
                     if (out_f32) {
-                        float* dst = reinterpret_cast<float*>(c) + (int64_t)row * ldc + col;
+                        float* dst = reinterpret_cast<float*>(c) + (int64_t)row * ldc + (int64_t)head * batch.c_cols + col;
 #pragma unroll
                         for (int e = 0; e < 32; e += 4)
                             if (col + e < N)
                                 *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]),
                                                                                   __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
                     } else {
-                        bf16* dst = reinterpret_cast<bf16*>(c) + (int64_t)row * ldc + col;
+                        bf16* dst = reinterpret_cast<bf16*>(c) + (int64_t)row * ldc + (int64_t)head * batch.c_cols + col;
 #pragma unroll
                         for (int e = 0; e < 32; e += 8)
                             if (col + e < N) {
@@ -513,13 +530,13 @@ GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, i
     if (attr_set_dev != DeviceOnce::SET) {
         cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
+            e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
         attr_set.mark(attr_set_dev);
     }
     if (persistent) {
-        GLMB_LAUNCH(gemm_bf16_tcgen05_persistent_kernel, dim3(total2 < sm_count ? total2 : sm_count), TC_THREADS, T2_SMEM_BYTES,
-                    (cudaStream_t)stream, map_a, map_b, c, ldc, rows, N, K, (const TcTile*)tiles, n_tiles, max_tiles, out_f32, status, no_allreduce());
+        GLMB_LAUNCH(gemm_bf16_tcgen05_persistent_kernel<false>, dim3(total2 < sm_count ? total2 : sm_count), TC_THREADS, T2_SMEM_BYTES,
+                    (cudaStream_t)stream, map_a, map_b, c, ldc, rows, N, K, (const TcTile*)tiles, n_tiles, max_tiles, out_f32, status, no_allreduce(), GemmBatch());
         return (int)cudaGetLastError();
     }
     dim3 grid(ceil_div(N, TC_BN), m_tiles);
@@ -549,7 +566,7 @@ GLMB_API int glmb_gemm_bf16_tcgen05_allreduce(const void* a, int64_t lda, const 
     static DeviceOnce attr_set;
     const int attr_set_dev = attr_set.pending();
     if (attr_set_dev != DeviceOnce::SET) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
         attr_set.mark(attr_set_dev);
     }
@@ -563,8 +580,8 @@ GLMB_API int glmb_gemm_bf16_tcgen05_allreduce(const void* a, int64_t lda, const 
     ar.out_offset = out_offset;
     ar.comm = *comm;
     void* c = comm->data[comm->rank] + out_offset;
-    GLMB_LAUNCH(gemm_bf16_tcgen05_persistent_kernel, dim3(total < sm_count ? total : sm_count), TC_THREADS, T2_SMEM_BYTES, (cudaStream_t)stream,
-                map_a, map_b, c, (int64_t)N, rows, N, K, (const TcTile*)nullptr, (const int*)nullptr, 0, 0, status, ar);
+    GLMB_LAUNCH(gemm_bf16_tcgen05_persistent_kernel<false>, dim3(total < sm_count ? total : sm_count), TC_THREADS, T2_SMEM_BYTES, (cudaStream_t)stream,
+                map_a, map_b, c, (int64_t)N, rows, N, K, (const TcTile*)nullptr, (const int*)nullptr, 0, 0, status, ar, GemmBatch());
     return (int)cudaGetLastError();
 }
 
@@ -594,4 +611,37 @@ GLMB_API int glmb_gemm_gated_takes(int rows, int N, int K) {
     gemm_pair_columns(rows, 2 * N, &plain);
     const int gated = 100 * ceil_div(ceil_div(rows, 256) * ceil_div(N, 128), 74);
     return (gated - plain) * (0.246 * K / 4096) < 2.0 + (double)rows * N * 6 / 4.5e6;
+}
+
+// `heads` products side by side: c[rows, h c_cols ..] (N columns, bf16) = a[rows, h a_cols ..] (K columns) . B_h, where B_h^T is [N, K] in rows
+// h b_rows + b_row0 .. of b (by_k = 0), or B_h is [K, N] there (by_k = 1).  b has heads * b_rows rows.  K a multiple of 64, N and every
+// offset and leading dimension multiples of 8, operands 16-byte aligned.
+GLMB_API int glmb_gemm_bf16_heads(const void* a, int64_t lda, int a_cols, const void* b, int64_t ldb, int b_rows, int b_row0, int by_k, void* c, int64_t ldc,
+                                  int c_cols, int heads, int rows, int N, int K, uint32_t* status, void* stream) {
+    if (rows < 1 || heads < 1 || N < 8 || (N & 7) || K < 64 || (K & 63) || (lda & 7) || (ldb & 7) || (ldc & 7) || (a_cols & 7) || (c_cols & 7)) return 1;
+    if (b_row0 < 0 || b_rows < b_row0 + (by_k ? K : N)) return 1;
+    if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) return 1;
+    CUtensorMap map_a, map_b;
+    if (make_map(&map_a, a, (uint64_t)rows, (uint64_t)(heads - 1) * a_cols + K, (uint64_t)lda)) return 3;
+    if (make_map(&map_b, b, (uint64_t)heads * b_rows, (uint64_t)(by_k ? N : K), (uint64_t)ldb, by_k ? 64 : T2_BN)) return 3;
+    static DeviceOnce once;
+    const int dev = once.pending();
+    if (dev != DeviceOnce::SET) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(gemm_bf16_tcgen05_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        once.mark(dev);
+    }
+    GemmBatch batch;
+    batch.count = heads; batch.a_cols = a_cols; batch.b_rows = b_rows; batch.b_row0 = b_row0; batch.c_cols = c_cols;
+    const int64_t total = (int64_t)heads * ceil_div(rows, TC_BM) * ceil_div(N, T2_BN);
+    if (total > 1 << 30) return 2;
+#define CALL(MN)                                                                                                                              \
+    GLMB_LAUNCH(gemm_bf16_tcgen05_persistent_kernel<MN>, (int)(total < 148 ? total : 148), TC_THREADS, T2_SMEM_BYTES, (cudaStream_t)stream, map_a, map_b, c, \
+                ldc, rows, N, K, (const TcTile*)nullptr, (const int*)nullptr, 0, 0, status, no_allreduce(), batch)
+    if (by_k) CALL(true);
+    else CALL(false);
+#undef CALL
+    return (int)cudaGetLastError();
 }

@@ -300,6 +300,14 @@ class GlmMoeDsaModel:
         g32, u32 = gate.float(), up.float()  # odd shapes of fixtures only
         return (g32 * torch.sigmoid(g32) * u32).to(torch.bfloat16)
 
+    def _heads_gemm(self, rows: int, kv_b: torch.Tensor) -> bool:
+        """Whether the per-head products of a prefill chunk (absorbed query, value projection) take the batched tcgen05 GEMM, which reads
+        queries and writes results where they lie; the library's form copies both (2,048 rows of 64 heads: 157 us each, 120 of them copies, against
+        71 and 47 us).  Few rows keep the library's form and their recorded launch program."""
+        g = self.g
+        return (rows > 256 and g.qk_nope_head_dim % 64 == 0 and g.kv_lora_rank % 64 == 0 and g.v_head_dim % 8 == 0 and g.kv_row_width % 8 == 0
+                and kv_b.is_contiguous() and kv_b.data_ptr() % 16 == 0)
+
     def _gated(self, x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
         """``bf16(g * sigmoid(g) * u)`` of a prefill chunk's gate and up projections: one launch where that is the faster form."""
         if (native.gemm_gated_takes(x.shape[0], gate.shape[0], x.shape[1]) and gate.stride() == up.stride()
@@ -383,9 +391,13 @@ class GlmMoeDsaModel:
             if gather and not xf:
                 self._allgather_heads(ws.q_full[:rows])
         else:
-            w_k = lw.kv_b[:, : g.qk_nope_head_dim, :]  # [hl, nope, L]
-            q_c = torch.einsum("rhd,hdc->rhc", ws.q_nope[:rows], w_k)
-            ws.q_full[:rows, hb : hb + hl, :L] = q_c
+            if self._heads_gemm(rows, lw.kv_b):
+                native.gemm_bf16_heads(ws.q_nope[:rows], lw.kv_b, 0, True, ws.q_full[:rows, hb : hb + hl], N=L, K=g.qk_nope_head_dim,
+                                       status=self.peer.status_ptr)
+            else:
+                w_k = lw.kv_b[:, : g.qk_nope_head_dim, :]  # [hl, nope, L]
+                q_c = torch.einsum("rhd,hdc->rhc", ws.q_nope[:rows], w_k)
+                ws.q_full[:rows, hb : hb + hl, :L] = q_c
             if gather:
                 self._allgather_heads(ws.q_full[:rows])
 
@@ -440,8 +452,13 @@ class GlmMoeDsaModel:
                 native.skinny_bf16(ws.attn_v[:rows], lw.w_o, ws.partial, native.SK_OUT_F32)
                 ws.attn_out[:rows] = self._allreduce_rows(ws.partial[:rows]).to(torch.bfloat16)
         else:
-            w_v = lw.kv_b[:, g.qk_nope_head_dim :, :]  # [hl, v, L]
-            v = torch.einsum("rhc,hvc->rhv", ws.o_lat[:rows], w_v).reshape(rows, hl * g.v_head_dim)
+            if self._heads_gemm(rows, lw.kv_b):
+                v = torch.empty((rows, hl * g.v_head_dim), dtype=torch.bfloat16, device=self.device)
+                native.gemm_bf16_heads(ws.o_lat[:rows], lw.kv_b, g.qk_nope_head_dim, False, v.view(rows, hl, g.v_head_dim), N=g.v_head_dim, K=L,
+                                       status=self.peer.status_ptr)
+            else:
+                w_v = lw.kv_b[:, g.qk_nope_head_dim :, :]  # [hl, v, L]
+                v = torch.einsum("rhc,hvc->rhv", ws.o_lat[:rows], w_v).reshape(rows, hl * g.v_head_dim)
             if self.world == 1:
                 self._mm(v, lw.w_o, out=ws.attn_out[:rows])
             else:

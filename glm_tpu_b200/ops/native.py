@@ -921,3 +921,14 @@ def gemm_bf16_gated(a, gate, up, out, kind, *, status=None):
                                    rows, gate.shape[0], K, int(kind), _p(status), _stream()),
         "gemm_bf16_gated",
     )
+
+
+def gemm_bf16_heads(a, b, b_row0: int, by_k: bool, out, *, N: int, K: int, status=None):
+    """``out[:, h, :N] = a[:, h, :K] @ B_h`` for every head ``h`` in one launch: ``a`` ``[rows, heads, >= K]`` and ``out`` ``[rows, heads, >= N]`` bf16 with
+    contiguous last axes, ``b`` contiguous ``[heads, R, C]`` whose rows ``b_row0 ..`` are ``B_h`` itself (``by_k``: K rows of N) or its transpose (N rows of K)."""
+    rows, heads = a.shape[:2]
+    _check(
+        lib().glmb_gemm_bf16_heads(_p(a), C.c_int64(a.stride(0)), a.stride(1), _p(b), C.c_int64(b.stride(1)), b.shape[1], int(b_row0), int(by_k), _p(out),
+                                   C.c_int64(out.stride(0)), out.stride(1), heads, rows, N, K, _p(status), _stream()),
+        "gemm_bf16_heads",
+    )
