@@ -1315,9 +1315,15 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
             }
         // routed gate/up of this GPU's routes: one item = (route, 16 output rows), moe_gateup_fp8_mma_kernel<1>
         {
-            bf16* x_sm = reinterpret_cast<bf16*>(big);  // the normalised rows, staged once (two resident CTAs leave almost no L1)
-            const size_t x_bytes = (mg_stage_rows(x_sm, a.x, H, rows, H) + 15) & ~(size_t)15;
-            float(*red)[2][MG_MM_ROWS][8] = reinterpret_cast<float(*)[2][MG_MM_ROWS][8]>(big + x_bytes);
+            // the normalised rows, staged once behind the sums (two resident CTAs leave almost no L1); eight wide rows do not fit beside them
+            // in the persistent kernel's region and are read where they are
+            float(*red)[2][MG_MM_ROWS][8] = reinterpret_cast<float(*)[2][MG_MM_ROWS][8]>(big);
+            constexpr size_t red_bytes = sizeof(float) * MG_WARPS * 2 * MG_MM_ROWS * 8;
+            const bf16* x_sm = a.x;
+            if (red_bytes + (size_t)rows * H * 2 <= (size_t)sm.big_bytes) {
+                mg_stage_rows(reinterpret_cast<bf16*>(big + red_bytes), a.x, H, rows, H);
+                x_sm = reinterpret_cast<const bf16*>(big + red_bytes);
+            }
             const int I = a.I, blocks = (I + MG_MM_ROWS - 1) / MG_MM_ROWS;
             const int items = sm.n_loc * blocks;
             const int g = lane >> 2, t = lane & 3;
@@ -1893,6 +1899,8 @@ GLMB_API int glmb_mega_supported(const MegaArgs* a) {
 // copy of the argument block (checked here), `device_args` the same bytes in device memory, which is what the kernel reads.
 GLMB_API int glmb_mega_decode(const MegaArgs* args, const void* device_args, int layer0, int phase0, int layer1, int phase1, void* stream) {
     if (glmb_mega_supported(args) || !device_args) return 1;
+    // the balanced projections keep their sums behind the step's rows: room for two weight rows at least
+    if (args->compat_ksplit != 1 && (size_t)args->rows * args->H * 2 + sizeof(float) * 2 * (MG_WARPS + 1) * GLMB_MAX_ROWS + 16 > MG_BIG_BYTES) return 1;
     if (layer0 < 0 || layer1 > args->num_layers || layer0 > layer1 || phase0 < 1 || phase1 < 1) return 1;
     const MegaArgs* d = reinterpret_cast<const MegaArgs*>(device_args);
     cudaStream_t st = (cudaStream_t)stream;
