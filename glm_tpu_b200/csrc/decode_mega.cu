@@ -445,7 +445,16 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int 
                     for (int r = 0; r < R; ++r) sm.red[warp][j][r] = acc[j][r];
             }
             __syncthreads();
-            if (kpart == 0 && lane == 0) {
+            if (mma) {
+                if (warp == 0 && lane == 0) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int r = 0; r < R; ++r)  // in pairs, as skm_sum
+                            acc[j][r] = ((acc[j][r] + sm.red[1][j][r]) + (sm.red[2][j][r] + sm.red[3][j][r])) +
+                                        ((sm.red[4][j][r] + sm.red[5][j][r]) + (sm.red[6][j][r] + sm.red[7][j][r]));
+                }
+            } else if (kpart == 0 && lane == 0) {
                 for (int p = 1; p < ks; ++p)
 #pragma unroll
                     for (int j = 0; j < 2; ++j)

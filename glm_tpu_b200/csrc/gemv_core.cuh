@@ -84,15 +84,28 @@ __device__ __forceinline__ void warp_reduce_all(float (&acc)[NPW][R]) {
 // instruction whatever R is, and nothing is shuffled at the end.  Measured on a B200, [6144 x 16384]: 2 rows 49.8 -> 32.2 us, 4 rows
 // 58.0 -> 32.6, 8 rows 85.5 -> 32.9 (6.1 TB/s); [131072 x 4096]: 193 -> 154, 218 -> 158, 397 -> 163.
 //
+// The tensor core truncates what it adds to an accumulator, so every instruction starts from zero and its sixteen products' sum is added in
+// rounded fp32: the four sums of a chunk in pairs, the chunk's to the warp's with Kahan's compensation, the warps' in pairs.  Error against
+// 64 bits (2-norm, operands of either sign), [6144 x 16384] / [6144 x 6144] / [2048 x 2048]: 7.3e-8 / 7.1e-8 / 7.1e-8, with FMAs 12.6e-8 /
+// 9.2e-8 / 7.5e-8, accumulated inside the tensor core 2.1e-6 / 7.3e-7 / 2.3e-7.  The additions hide behind the loads: [6144 x 16384] 31.6 ->
+// 32.0 us, [4096 x 18432] 24.7 -> 25.0, [131072 x 4096] 154 -> 156.
+//
 // The k index inside an instruction is a permutation of the true k, the same for both operands: lane (g, t) holds 16 consecutive
 // k values of weight rows g (w_lo) and g + 8 (w_hi) and of activation row g, at 16 t of a 64-wide chunk, so every load is a full
 // 16-byte vector.  Chunks first, first + stride, .. enter the sum in ascending order, whatever DEPTH (chunks whose loads are in
 // flight together) is.  `skinny_mma_span`: the SKM_WARPS warps of a CTA take the chunks of K round-robin; the bits depend on K only.
 // w_lo, w_hi, xr: this lane's rows (NULL: zeros).  K a multiple of 8.  c: the C fragment, rows g and g + 8, columns 2t and 2t + 1.
 #define SKM_WARPS 8
+// d = a . b, the sums of sixteen products
+__device__ __forceinline__ void mma_16816_alone(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 template <int DEPTH>
 __device__ __forceinline__ void skinny_mma_chunks(const bf16* w_lo, const bf16* w_hi, const bf16* xr, int K, int first, int stride, int chunks, int t,
                                                   float (&c)[4]) {
+    float lost[4] = {0.f, 0.f, 0.f, 0.f};
     for (int c0 = first; c0 < chunks; c0 += stride * DEPTH) {
         uint4 lo[DEPTH][2], hi[DEPTH][2], x[DEPTH][2];
 #pragma unroll
@@ -106,12 +119,20 @@ __device__ __forceinline__ void skinny_mma_chunks(const bf16* w_lo, const bf16* 
                 x[u][h] = xr && k < K ? ld_hot16(xr + k) : zero;
             }
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u)
+        for (int u = 0; u < DEPTH; ++u) {
+            float d[2][2][4];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                mma_16816(c, lo[u][h].x, hi[u][h].x, lo[u][h].y, hi[u][h].y, x[u][h].x, x[u][h].y);
-                mma_16816(c, lo[u][h].z, hi[u][h].z, lo[u][h].w, hi[u][h].w, x[u][h].z, x[u][h].w);
+                mma_16816_alone(d[h][0], lo[u][h].x, hi[u][h].x, lo[u][h].y, hi[u][h].y, x[u][h].x, x[u][h].y);
+                mma_16816_alone(d[h][1], lo[u][h].z, hi[u][h].z, lo[u][h].w, hi[u][h].w, x[u][h].z, x[u][h].w);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float part = ((d[0][0][i] + d[0][1][i]) + (d[1][0][i] + d[1][1][i])) - lost[i], sum = c[i] + part;
+                lost[i] = (sum - c[i]) - part;
+                c[i] = sum;
+            }
+        }
     }
 }
 template <int DEPTH>
@@ -139,10 +160,8 @@ __device__ __forceinline__ void skm_store_fragment(float* red, const float (&c)[
     red[(2 * t) * SKM_RED + g] = c[0]; red[(2 * t + 1) * SKM_RED + g] = c[1];
     red[(2 * t) * SKM_RED + g + 8] = c[2]; red[(2 * t + 1) * SKM_RED + g + 8] = c[3];
 }
-// Sum over the warps' K parts of (activation row r, weight row n), in warp order.
+// Sum over the warps' K parts of (activation row r, weight row n), in pairs.
 __device__ __forceinline__ float skm_sum(const float (*red)[8 * SKM_RED], int r, int n) {
-    float s = red[0][r * SKM_RED + n];
-#pragma unroll
-    for (int p = 1; p < SKM_WARPS; ++p) s += red[p][r * SKM_RED + n];
-    return s;
+    const int at = r * SKM_RED + n;
+    return ((red[0][at] + red[1][at]) + (red[2][at] + red[3][at])) + ((red[4][at] + red[5][at]) + (red[6][at] + red[7][at]));
 }

@@ -48,3 +48,22 @@ def test_gated_projection(rows, N, K):
     want = g * torch.sigmoid(g) * u
     # either factor may land on the neighbouring bf16 (2^-8), the gate's slope is at most 1.1, and the result is rounded once more
     assert ((act.float() - want).abs() <= 2**-6 * want.abs() + 2**-8 * u.abs() * 1.1 * g.abs().clamp_min(2**-8)).all()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8])
+@pytest.mark.parametrize("N,K", [(1009, 200), (2048, 2048), (6144, 6144), (6144, 16384)])
+@pytest.mark.parametrize("sign", [0, 1])
+def test_sums_are_as_exact_as_fp32_additions(rows, N, K, sign):
+    """2-norm of the error: whatever K is, about that of a few additions."""
+    from glm_tpu_b200.ops import native as n
+
+    x, w = _bf16((rows, K), rows + K), _bf16((N, K), N, 0.1)
+    if sign:  # nothing cancels: an accumulator that truncates loses something in every step
+        x, w = x.abs(), w.abs()
+    out = torch.empty(rows, N, device="cuda")
+    n.skinny_bf16(x, w, out, n.SK_OUT_F32)
+    want = x.double() @ w.double().T
+    err = float((out.double() - want).norm() / want.norm())
+    # parts of n random products out of K are off by u sqrt(n / K) of the result when added, u = 2^-24 / sqrt(3) at most: eight warps in pairs 3 u^2, a warp's own
+    # sum 1, the four sums of a chunk 2.5 (where nothing cancels the parts are n / K, less); sixteen products alone are truncated, 2^-24
+    assert err <= 2.0**-24 * (1 + (6.5 / 3) ** 0.5)
