@@ -175,11 +175,16 @@ struct MgSmall {
     MegaLayer layer;  // the pointer-table entry of the layer in progress
     float red[MG_WARPS][2][GLMB_MAX_ROWS];
     float sh[GLMB_AR_SLICE];
-    float scratch[3][40];
-    float s_key[256];
-    unsigned long long best[MG_WARPS][GLMB_MAX_ROWS];
-    int ids[GLMB_MAX_ROWS][MG_MAX_TOPK];
-    float wts[GLMB_MAX_ROWS][MG_MAX_TOPK];
+    union {
+        struct {
+            float scratch[3][40];
+            float s_key[256];
+            unsigned long long best[MG_WARPS][GLMB_MAX_ROWS];
+            int ids[GLMB_MAX_ROWS][MG_MAX_TOPK];
+            float wts[GLMB_MAX_ROWS][MG_MAX_TOPK];
+        };
+        float frag[MG_WARPS][16][GLMB_MAX_ROWS];  // mg_gemv_mma: sums of the warps (none of the others lives across a projection)
+    };
     int loc[GLMB_MAX_ROWS * MG_MAX_TOPK];
     float w_s[MG_MERGE_MAX_CHUNKS];
     float red_s[8];
@@ -314,11 +319,8 @@ __device__ __forceinline__ int mg_pick_ks(int units, int K, bool compat, int max
     return best;
 }
 
-// The compatible split of a projection of `rows16` groups of 16 weight rows (a gate / up pair: 8 + 8) and `units` pairs, as the stand-alone
-// kernels add: all warps (mg_gemv's `mma`), or the split of skinny_bf16_kernel for one row and few outputs.
-__device__ __forceinline__ int mg_split(int rows, int rows16, int units, int K) {
-    return rows > 1 && skinny_mma_takes(rows16) ? SKM_WARPS : mg_pick_ks(units, K, true, 0, 0);
-}
+// Whether a projection of `rows16` groups of 16 weight rows (a gate / up pair: 8 + 8) takes mg_gemv_mma, as the stand-alone kernels do.
+__host__ __device__ static inline bool mg_takes_mma(int rows, int rows16) { return rows > 1 && skinny_mma_takes(rows16); }
 
 // warp_dot_bf16 (gemv_core.cuh) with U steps of loads issued before their arithmetic: the same products added in the same
 // order, but 2 * U 16-byte loads in flight per lane, which the 16 resident warps of an SM need to keep HBM busy.
@@ -394,23 +396,39 @@ struct MgUnit {
     const bf16* w1;
 };
 
-// The sums of a unit's two weight rows with the mma inner loop of the stand-alone kernels (the two rows are rows 0 and 1 of the
-// 16-row fragment, the others zero: an output of mma.sync depends on its own row and column only); the first lane gets acc.
-template <int R>
-__device__ __forceinline__ void mg_warp_mma(const MgUnit& m, int K, int rows, int warp, int lane, float (&acc)[2][R]) {
-    const int g = lane >> 2, t = lane & 3;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    skinny_mma_span<2>(g == 0 ? m.w0 : g == 1 ? m.w1 : nullptr, nullptr, g < rows ? m.x + (int64_t)g * m.xs : nullptr, K, warp, t, c);
+// Units of two weight rows with the mma inner loop of the stand-alone kernels: a CTA takes eight units at a time, their first rows over their
+// second rows as a fragment, its warps split K, and the first lane of warp w hands the R x 2 sums of unit w to `epi(unit, round, w, acc)`.  A step of
+// four GLM-5.3 layers in phases: two lanes 2,346 us (a unit per fragment, 8 of 32 lanes loading: 4,000), four 2,787 (4,378), eight 3,766 (7,174).
+#define MG_MMA_UNITS 8
+template <int R, typename Get, typename Epi>
+__device__ __forceinline__ void mg_gemv_mma(int units, int K, int rows, MgSmall& sm, Get get, Epi epi) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    for (int it = 0, u0 = (int)blockIdx.x * MG_MMA_UNITS; u0 < units; ++it, u0 += (int)gridDim.x * MG_MMA_UNITS) {
+        const bool own = u0 + g < units;
+        const MgUnit m = get(own ? u0 + g : u0);
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        skinny_mma_span<(R <= 4 ? 2 : 4)>(own ? m.w0 : nullptr, own ? m.w1 : nullptr, g < rows ? m.x + (int64_t)g * m.xs : nullptr, K, warp, t, c);
+        __syncthreads();  // the sums of the round before have been read
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+        for (int q = 0; q < 4; ++q)
+            if (2 * t + (q & 1) < R) sm.frag[warp][g + 8 * (q >> 1)][2 * t + (q & 1)] = c[q];
+        __syncthreads();
+        const int j = lane / R & 1, r = lane % R;
+        float part[MG_WARPS];
 #pragma unroll
-        for (int r = 0; r < R; ++r) acc[j][r] = __shfl_sync(0xffffffffu, c[r & 1], j * 4 + (r >> 1));
+        for (int w = 0; w < MG_WARPS; ++w) part[w] = sm.frag[w][warp + 8 * j][r];
+        const float v = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));  // in pairs, as skm_sum
+        float acc[2][R];
+#pragma unroll
+        for (int i = 0; i < 2 * R; ++i) acc[i / R][i % R] = __shfl_sync(0xffffffffu, v, i);
+        if (lane == 0 && u0 + warp < units) epi(u0 + warp, it, warp, acc);
+    }
 }
 
 // Units of two weight rows over the whole grid: a team of `ks` warps of one CTA owns a unit, splits K, and its first
-// lane hands the R x 2 sums to `epi(unit, acc)`.  mma: with mg_warp_mma (ks == SKM_WARPS).
+// lane hands the R x 2 sums to `epi(unit, round, team, acc)`.
 template <int R, typename Get, typename Epi>
-__device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int rows, MgSmall& sm, Get get, Epi epi) {
+__device__ __forceinline__ void mg_gemv(int units, int K, int ks, int rows, MgSmall& sm, Get get, Epi epi) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tpc = MG_WARPS / ks, team = warp / ks, kpart = warp % ks;
     const int total_teams = gridDim.x * tpc;
@@ -425,16 +443,12 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int 
             for (int r = 0; r < R; ++r) acc[j][r] = 0.f;
         if (u < units) {
             const MgUnit m = get(u);
-            if (mma) {
-                mg_warp_mma<R>(m, K, rows, warp, lane, acc);
-            } else {
-                const bf16* xr[R];
+            const bf16* xr[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) xr[r] = m.x + (int64_t)(r < rows ? r : 0) * m.xs;
-                const bf16* wp[2] = {m.w0, m.w1};
-                mg_warp_dot<R, (R <= 2 ? 8 : (R <= 4 ? 4 : 2))>(xr, wp, kpart * kspan, (kpart + 1) * kspan, lane, acc);
-                warp_reduce_all<R, 2>(acc);
-            }
+            for (int r = 0; r < R; ++r) xr[r] = m.x + (int64_t)(r < rows ? r : 0) * m.xs;
+            const bf16* wp[2] = {m.w0, m.w1};
+            mg_warp_dot<R, (R <= 2 ? 8 : (R <= 4 ? 4 : 2))>(xr, wp, kpart * kspan, (kpart + 1) * kspan, lane, acc);
+            warp_reduce_all<R, 2>(acc);
         }
         if (ks > 1) {
             __syncthreads();
@@ -445,16 +459,7 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int 
                     for (int r = 0; r < R; ++r) sm.red[warp][j][r] = acc[j][r];
             }
             __syncthreads();
-            if (mma) {
-                if (warp == 0 && lane == 0) {
-#pragma unroll
-                    for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int r = 0; r < R; ++r)  // in pairs, as skm_sum
-                            acc[j][r] = ((acc[j][r] + sm.red[1][j][r]) + (sm.red[2][j][r] + sm.red[3][j][r])) +
-                                        ((sm.red[4][j][r] + sm.red[5][j][r]) + (sm.red[6][j][r] + sm.red[7][j][r]));
-                }
-            } else if (kpart == 0 && lane == 0) {
+            if (kpart == 0 && lane == 0) {
                 for (int p = 1; p < ks; ++p)
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
@@ -464,6 +469,13 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, bool mma, int 
         }
         if (kpart == 0 && lane == 0 && u < units) epi(u, it, team, acc);
     }
+}
+
+// A projection of `rows16` groups of 16 weight rows with the sums of the stand-alone kernels.
+template <int R, typename Get, typename Epi>
+__device__ __forceinline__ void mg_project(int rows16, int units, int K, int rows, MgSmall& sm, Get get, Epi epi) {
+    if (mg_takes_mma(rows, rows16)) mg_gemv_mma<R>(units, K, rows, sm, get, epi);
+    else mg_gemv<R>(units, K, mg_pick_ks(units, K, true, 0, 0), rows, sm, get, epi);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -648,9 +660,9 @@ template <int R>
 __device__ __forceinline__ void mg_gemv_allreduce(const bf16* x, int64_t xs, const bf16* w, int64_t ws, int N, int K, int rows, bf16* out,
                                                   int64_t os, int channel, const MegaArgs& a, MgSmall& sm) {
     const int units = (N + 1) / 2;
-    const bool mma = rows > 1 && a.comm.world == 1 && skinny_mma_takes((N + 15) / 16);  // the exchange of several GPUs stays with the FMA kernel (glmb_skinny_bf16)
-    const int ks = mma ? SKM_WARPS : mg_pick_ks(units, K, true, GLMB_AR_SLICE, 2 * R);
-    const int tpc = MG_WARPS / ks;
+    const bool mma = a.comm.world == 1 && mg_takes_mma(rows, (N + 15) / 16);  // the exchange of several GPUs stays with the FMA kernel (glmb_skinny_bf16)
+    const int ks = mma ? 0 : mg_pick_ks(units, K, true, GLMB_AR_SLICE, 2 * R);
+    const int tpc = mma ? MG_MMA_UNITS : MG_WARPS / ks;
     const int total_teams = gridDim.x * tpc;
     const int rounds = (units + total_teams - 1) / total_teams;
     const int per_round = tpc * 2 * R;
@@ -658,17 +670,18 @@ __device__ __forceinline__ void mg_gemv_allreduce(const bf16* x, int64_t xs, con
         if (threadIdx.x == 0 && blockIdx.x == 0) raise_status(a.status, GLMB_STATUS_BAD_SHAPE);
         return;
     }
-    mg_gemv<R>(units, K, ks, mma, rows, sm,
-               [&](int u) {
-                   const int n0 = u * 2;
-                   return MgUnit{x, xs, w + (int64_t)n0 * ws, w + (int64_t)min(n0 + 1, N - 1) * ws};
-               },
-               [&](int, int it, int team, float (&acc)[2][R]) {
+    auto get = [&](int u) {
+        const int n0 = u * 2;
+        return MgUnit{x, xs, w + (int64_t)n0 * ws, w + (int64_t)min(n0 + 1, N - 1) * ws};
+    };
+    auto keep = [&](int, int it, int team, float (&acc)[2][R]) {
 #pragma unroll
-                   for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-                       for (int r = 0; r < R; ++r) sm.sh[it * per_round + (team * 2 + j) * R + r] = acc[j][r];
-               });
+            for (int r = 0; r < R; ++r) sm.sh[it * per_round + (team * 2 + j) * R + r] = acc[j][r];
+    };
+    if (mma) mg_gemv_mma<R>(units, K, rows, sm, get, keep);
+    else mg_gemv<R>(units, K, ks, rows, sm, get, keep);
     // a CTA whose every unit is past the end has nothing to exchange (the same CTAs on every rank)
     const int first_unit = (int)blockIdx.x * tpc;
     if (first_unit >= units) return;
@@ -1009,8 +1022,7 @@ __device__ MG_CALL void mg_qkv_a(const MegaArgs& a, const MegaLayer& lw, int lay
                               [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.proj_a, a.proj_stride, rows, p0, cnt, vals); });
             return;
         }
-        const int ks = mg_split(rows, (N + 15) / 16, units, H);
-        mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
+        mg_project<R>((N + 15) / 16, units, H, rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{x_s, H, lw.w_qkv_a + (int64_t)n0 * H, lw.w_qkv_a + (int64_t)min(n0 + 1, N - 1) * H};
@@ -1063,8 +1075,7 @@ __device__ MG_CALL void mg_q_b(const MegaArgs& a, const MegaLayer& lw, int layer
                               [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.q_proj, a.q_stride, rows, p0, cnt, vals); });
             return;
         }
-        const int ks = mg_split(rows, (N + 15) / 16, units, Q);
-        mg_gemv<R>(units, Q, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
+        mg_project<R>((N + 15) / 16, units, Q, rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{q_s, Q, lw.w_q_b + (int64_t)n0 * Q, lw.w_q_b + (int64_t)min(n0 + 1, N - 1) * Q};
@@ -1190,7 +1201,7 @@ __device__ MG_CALL void mg_vproj(const MegaArgs& a, const MegaLayer& lw, int lay
         const int units = hl * per_head;
         const int ks = mg_pick_ks(per_head * hl, L, compat, 0, 0);
         const int64_t head_rows = (int64_t)(a.nope + vd) * L;
-        mg_gemv<R>(units, L, ks, false, rows, sm,
+        mg_gemv<R>(units, L, ks, rows, sm,
                    [&](int u) {
                        const int h = u / per_head, n0 = (u % per_head) * 2;
                        const bf16* wv = lw.kv_b + h * head_rows + (int64_t)a.nope * L;
@@ -1244,8 +1255,7 @@ __device__ MG_CALL void mg_mlp_a(const MegaArgs& a, const MegaLayer& lw, int lay
                                   });
                 return;
             }
-            const int ks = mg_split(rows, (N + 7) / 8, N, H);
-            mg_gemv<R>(N, H, ks, rows > 1 && skinny_mma_takes((N + 7) / 8), rows, sm,
+            mg_project<R>((N + 7) / 8, N, H, rows, sm,
                        [&](int u) { return MgUnit{x_s, H, wg + (int64_t)u * H, wu + (int64_t)u * H}; },
                        [&](int u, int, int, float (&acc)[2][R]) {
 #pragma unroll
@@ -1266,8 +1276,7 @@ __device__ MG_CALL void mg_mlp_a(const MegaArgs& a, const MegaLayer& lw, int lay
                 swiglu(lw.shared_gate, lw.shared_up, a.shared_cols, a.act_shared, a.act_shared_stride);
                 return;
             }
-            const int ks = mg_split(rows, (E + 15) / 16, units, H);
-            mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((E + 15) / 16), rows, sm,
+            mg_project<R>((E + 15) / 16, units, H, rows, sm,
                        [&](int u) {
                            const int n0 = u * 2;
                            return MgUnit{x_s, H, lw.router_w + (int64_t)n0 * H, lw.router_w + (int64_t)min(n0 + 1, E - 1) * H};
@@ -1328,11 +1337,9 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
             // in the persistent kernel's region and are read where they are
             float(*red)[2][MG_MM_ROWS][8] = reinterpret_cast<float(*)[2][MG_MM_ROWS][8]>(big);
             constexpr size_t red_bytes = sizeof(float) * MG_WARPS * 2 * MG_MM_ROWS * 8;
-            const bf16* x_sm = a.x;
-            if (red_bytes + (size_t)rows * H * 2 <= (size_t)sm.big_bytes) {
-                mg_stage_rows(reinterpret_cast<bf16*>(big + red_bytes), a.x, H, rows, H);
-                x_sm = reinterpret_cast<const bf16*>(big + red_bytes);
-            }
+            bf16* x_sm = reinterpret_cast<bf16*>(big + red_bytes);
+            const bool staged = red_bytes + (size_t)rows * H * 2 <= (size_t)sm.big_bytes;
+            if (staged) mg_stage_rows(x_sm, a.x, H, rows, H);
             const int I = a.I, blocks = (I + MG_MM_ROWS - 1) / MG_MM_ROWS;
             const int items = sm.n_loc * blocks;
             const int g = lane >> 2, t = lane & 3;
@@ -1341,7 +1348,7 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
                 const int p = sm.loc[item / blocks], n0 = (item % blocks) * MG_MM_ROWS;
                 const int e = sm.ids[p / tk][p % tk] - a.expert_base;
                 const int route = g == 0 ? p : -1;
-                const bf16* xr = x_sm + (int64_t)(route >= 0 ? route / tk : 0) * H;
+                const int64_t x_row = (int64_t)(route >= 0 ? route / tk : 0) * H;
                 const uint8_t* wg_lo = lw.exp_gate + ((int64_t)e * I + n0 + g) * H;
                 const uint8_t* wu_lo = lw.exp_up + ((int64_t)e * I + n0 + g) * H;
                 const int64_t hi_off = (int64_t)8 * H;
@@ -1360,7 +1367,8 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
                             g_lo[u] = ld_stream16(wg_lo + k); g_hi[u] = ld_stream16(wg_lo + hi_off + k);
                             u_lo[u] = ld_stream16(wu_lo + k); u_hi[u] = ld_stream16(wu_lo + hi_off + k);
                             x0[u] = x1[u] = make_uint4(0, 0, 0, 0);
-                            if (route >= 0) { x0[u] = ld_hot16(xr + k); x1[u] = ld_hot16(xr + k + 8); }
+                            if (route >= 0 && staged) { x0[u] = ld_hot16(x_sm + x_row + k); x1[u] = ld_hot16(x_sm + x_row + k + 8); }
+                            if (route >= 0 && !staged) { x0[u] = ld_hot16(a.x + x_row + k); x1[u] = ld_hot16(a.x + x_row + k + 8); }
                             s_g[u] = lw.exp_gate_scale[sofs + (c >> 1)]; s_u[u] = lw.exp_up_scale[sofs + (c >> 1)];
                         }
                     }
@@ -1403,8 +1411,7 @@ __device__ MG_CALL void mg_mlp_b(const MegaArgs& a, const MegaLayer& lw, int lay
                                   [&](int p0, int cnt, const float* vals) { mg_store_f32<R>(a.partial, H, rows, p0, cnt, vals); });
                 return;
             }
-            const int ks = mg_split(rows, (H + 15) / 16, units, K);
-            mg_gemv<R>(units, K, ks, rows > 1 && skinny_mma_takes((H + 15) / 16), rows, sm,
+            mg_project<R>((H + 15) / 16, units, K, rows, sm,
                        [&](int u) {
                            const int n0 = u * 2;
                            return MgUnit{a.act_shared, a.act_shared_stride, lw.shared_down + (int64_t)n0 * K,
@@ -1557,7 +1564,6 @@ __device__ MG_CALL void mg_head_phase(const MegaArgs& a, int phase, MgSmall& sm,
         bf16* x_s = reinterpret_cast<bf16*>(big);
         mg_norm_rows(a, a.num_layers == 0 ? nullptr : a.update, a.residual_a, a.num_layers == 0, a.final_norm, x_s, nullptr, nullptr, sm);
         const int N = a.vocab_local, units = (N + 1) / 2;
-        const int ks = mg_split(rows, (N + 15) / 16, units, H);
         if (!COMPAT) {
             int nf;
             float* scratch = mg_scratch(big, (size_t)rows * H * 2, &nf);
@@ -1579,7 +1585,7 @@ __device__ MG_CALL void mg_head_phase(const MegaArgs& a, int phase, MgSmall& sm,
         unsigned long long run[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) run[r] = 0ull;
-        mg_gemv<R>(units, H, ks, rows > 1 && skinny_mma_takes((N + 15) / 16), rows, sm,
+        mg_project<R>((N + 15) / 16, units, H, rows, sm,
                    [&](int u) {
                        const int n0 = u * 2;
                        return MgUnit{x_s, H, a.lm_head + (int64_t)n0 * H, a.lm_head + (int64_t)min(n0 + 1, N - 1) * H};
@@ -1761,8 +1767,11 @@ __global__ void __launch_bounds__(MG_THREADS, MG_CTAS_PER_SM) decode_mega_kernel
 // which the persistent form gives up (two 100 KB CTAs per SM leave no L1, every phase starts on cold code), and the chain is
 // still 11 launches per layer instead of 17.  Before it waits for its predecessor, a projection kernel asks the L2 for its own
 // block of weight rows: the fetch overlaps the tail of the previous kernel.
-__device__ __forceinline__ void mg_prefetch_rows(const bf16* base, int N, int align, size_t row_bytes) {
+// The compatible form, whose grids leave room for the next kernels' CTAs, asks for no more than the stand-alone kernels do (SK_PREFETCH_LIMIT): what the
+// L2 cannot hold would be read twice.
+__device__ __forceinline__ void mg_prefetch_rows(const MegaArgs& a, const bf16* base, int N, int align, size_t row_bytes) {
     if (threadIdx.x != 0 || base == nullptr) return;
+    if (a.compat_ksplit == 1 && (size_t)N * row_bytes > ((size_t)48 << 20)) return;
     int rpc = (N + (int)gridDim.x - 1) / (int)gridDim.x;
     rpc = (rpc + align - 1) / align * align;
     const int n_begin = (int)blockIdx.x * rpc, n_cnt = min(N, n_begin + rpc) - n_begin;
@@ -1775,26 +1784,26 @@ __device__ __forceinline__ void mg_prefetch_rows(const bf16* base, int N, int al
 __device__ __forceinline__ void mg_prefetch_own(const MegaArgs& a, const MegaLayer& lw, int layer, int phase) {
     const size_t H2 = (size_t)a.H * 2;
     if (layer >= a.num_layers) {
-        if (phase == MG_HEAD_LOGITS) mg_prefetch_rows(a.lm_head, a.vocab_local, 1, H2);
+        if (phase == MG_HEAD_LOGITS) mg_prefetch_rows(a, a.lm_head, a.vocab_local, 1, H2);
         return;
     }
     switch (phase) {
-    case MG_QKV_A: mg_prefetch_rows(lw.w_qkv_a, lw.n_qkv_a, 1, H2); break;
-    case MG_Q_B: mg_prefetch_rows(lw.w_q_b, lw.n_q_b, 1, (size_t)a.Q * 2); break;
-    case MG_OPROJ: mg_prefetch_rows(lw.w_o, a.H, 1, (size_t)a.heads_local * a.vdim * 2); break;
+    case MG_QKV_A: mg_prefetch_rows(a, lw.w_qkv_a, lw.n_qkv_a, 1, H2); break;
+    case MG_Q_B: mg_prefetch_rows(a, lw.w_q_b, lw.n_q_b, 1, (size_t)a.Q * 2); break;
+    case MG_OPROJ: mg_prefetch_rows(a, lw.w_o, a.H, 1, (size_t)a.heads_local * a.vdim * 2); break;
     case MG_MLP_A:
         if (lw.dense) {
-            mg_prefetch_rows(lw.dense_gate, a.dense_cols, 1, H2);
-            mg_prefetch_rows(lw.dense_up, a.dense_cols, 1, H2);
+            mg_prefetch_rows(a, lw.dense_gate, a.dense_cols, 1, H2);
+            mg_prefetch_rows(a, lw.dense_up, a.dense_cols, 1, H2);
         } else {
-            mg_prefetch_rows(lw.router_w, a.E, 1, H2);
-            mg_prefetch_rows(lw.shared_gate, a.shared_cols, 1, H2);
-            mg_prefetch_rows(lw.shared_up, a.shared_cols, 1, H2);
+            mg_prefetch_rows(a, lw.router_w, a.E, 1, H2);
+            mg_prefetch_rows(a, lw.shared_gate, a.shared_cols, 1, H2);
+            mg_prefetch_rows(a, lw.shared_up, a.shared_cols, 1, H2);
         }
         break;
     case MG_MLP_B:
-        if (lw.dense) mg_prefetch_rows(lw.dense_down, a.H, 1, (size_t)a.dense_cols * 2);
-        else mg_prefetch_rows(lw.shared_down, a.H, 1, (size_t)a.shared_cols * 2);
+        if (lw.dense) mg_prefetch_rows(a, lw.dense_down, a.H, 1, (size_t)a.dense_cols * 2);
+        else mg_prefetch_rows(a, lw.shared_down, a.H, 1, (size_t)a.shared_cols * 2);
         break;
     default: break;
     }
@@ -1803,15 +1812,15 @@ __device__ __forceinline__ void mg_prefetch_own(const MegaArgs& a, const MegaLay
 // PHASE: 1..11 a layer's phases, 12 / 13 the head's two (a kernel per phase: its own registers, occupancy and code).
 // Resident CTAs per SM a phase kernel is compiled for: the streaming phases want many small CTAs (every byte of the table
 // requested at once), which bounds their registers; the tile phases keep the registers they need.
-template <int R, int PHASE>
+template <int R, bool COMPAT, int PHASE>
 struct MgPhaseBlocks {
     static constexpr bool streaming = PHASE == MG_QKV_A || PHASE == MG_Q_B || PHASE == MG_VPROJ || PHASE == MG_OPROJ || PHASE == MG_MLP_A ||
                                       PHASE == MG_MLP_B || PHASE == MG_COMBINE + MG_HEAD_LOGITS;
-    static constexpr int value = !streaming ? 2 : (R <= 2 ? 4 : (R <= 4 ? 3 : 2));
+    static constexpr int value = !streaming ? 2 : R > 4 ? 2 : (R > 2 || (COMPAT && R > 1)) ? 3 : 4;  // mg_gemv_mma: 80 registers
 };
 
 template <int R, bool COMPAT, int PHASE>
-__global__ void __launch_bounds__(MG_THREADS, (MgPhaseBlocks<R, PHASE>::value)) mega_phase_kernel(const __grid_constant__ MegaArgs args, const __grid_constant__ MegaLayer lwp,
+__global__ void __launch_bounds__(MG_THREADS, (MgPhaseBlocks<R, COMPAT, PHASE>::value)) mega_phase_kernel(const __grid_constant__ MegaArgs args, const __grid_constant__ MegaLayer lwp,
                                                                 int layer, int big_bytes) {
     constexpr int phase = PHASE > MG_COMBINE ? PHASE - MG_COMBINE : PHASE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1830,6 +1839,7 @@ __global__ void __launch_bounds__(MG_THREADS, (MgPhaseBlocks<R, PHASE>::value)) 
 GLMB_API size_t glmb_mega_args_sizeof(void) { return sizeof(MegaArgs); }
 GLMB_API size_t glmb_mega_layer_sizeof(void) { return sizeof(MegaLayer); }
 GLMB_API size_t glmb_mega_barrier_sizeof(void) { return sizeof(MegaBarrier); }
+static_assert(MG_CTAS_PER_SM * (((sizeof(MgSmall) + 15) & ~(size_t)15) + MG_BIG_BYTES + 1024) <= 228 * 1024, "the resident CTAs share an SM's memory");
 static size_t mega_smem_bytes(void) { return ((sizeof(MgSmall) + 15) & ~(size_t)15) + MG_BIG_BYTES; }
 
 static int g_mega_cooperative = 1;
@@ -1932,9 +1942,13 @@ GLMB_API int glmb_mega_decode(const MegaArgs* args, const void* device_args, int
 // One phase as a kernel of its own.  Grid and shared memory follow from the shapes alone, so every GPU of a box launches the
 // same grid (the exchanges inside the all-reduce phases pair CTA j of every rank).
 static size_t phase_big_bytes(const MegaArgs& a, const MegaLayer& lw, int layer, int phase, int Rt) {
-    const size_t xH = (size_t)a.rows * a.H * 2, scratch = 16384;
+    // The compatible projections keep nothing here but the step's rows: what shared memory does not take is L1, which the loads in flight need (a
+    // step of four GLM-5.3 layers, one lane: 1,412 us with the scratch of the balanced form beside the rows, 1,337 without; four lanes 2,829,
+    // 2,787).  Eight rows are one CTA per SM either way.
+    const bool compat = a.compat_ksplit == 1;
+    const size_t xH = (size_t)a.rows * a.H * 2, scratch = compat && Rt <= 4 ? 0 : 16384;
     if (layer >= a.num_layers) return phase == MG_HEAD_LOGITS ? xH + scratch : 16;
-    auto staged = [&](size_t K) { const size_t x = (size_t)a.rows * K * 2; return (x <= 65536 ? x : 0) + scratch + 8192; };
+    auto staged = [&](size_t K) { const size_t x = (size_t)a.rows * K * 2; return compat ? 16 : (x <= 65536 ? x : 0) + scratch + 8192; };
     switch (phase) {
     case MG_QKV_A: case MG_MLP_A: return xH + scratch;
     case MG_Q_B: return (size_t)a.rows * a.Q * 2 + scratch;
@@ -1944,7 +1958,7 @@ static size_t phase_big_bytes(const MegaArgs& a, const MegaLayer& lw, int layer,
     case MG_MLP_B: {
         if (lw.dense) return staged(a.dense_cols);
         const size_t gate_up = xH + 16 + sizeof(float) * MG_WARPS * 2 * MG_MM_ROWS * 8;
-        const size_t shared_down = (size_t)a.rows * a.shared_cols * 2 + scratch;
+        const size_t shared_down = compat ? 0 : (size_t)a.rows * a.shared_cols * 2 + scratch;
         return gate_up > shared_down ? gate_up : shared_down;
     }
     case MG_MOE_DOWN: {
@@ -1961,7 +1975,10 @@ static int host_pick_ks(int units, int K) {
     return ks;
 }
 // CTAs that give every unit of a projection its team of warps in one round (units: pairs of rows, or gate / up pairs)
-static int one_round(int units, int K) { return (units + MG_WARPS / host_pick_ks(units, K) - 1) / (MG_WARPS / host_pick_ks(units, K)); }
+static int one_round(int rows, int rows16, int units, int K) {
+    const int per_cta = mg_takes_mma(rows, rows16) ? MG_MMA_UNITS : MG_WARPS / host_pick_ks(units, K);
+    return (units + per_cta - 1) / per_cta;
+}
 
 static int phase_grid(const MegaArgs& a, const MegaLayer& lw, int layer, int phase, int sms, int per_sm) {
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
@@ -1969,19 +1986,21 @@ static int phase_grid(const MegaArgs& a, const MegaLayer& lw, int layer, int pha
     auto at_most = [&](int items) { return items < 1 ? 1 : (items < wide ? items : wide); };
     auto capped = [&](int ctas) { return ctas < 1 ? 1 : (ctas > GLMB_AR_MAX_CTAS ? GLMB_AR_MAX_CTAS : ctas); };
     const int H = a.H;
-    if (layer >= a.num_layers) return phase == MG_HEAD_LOGITS ? (a.compat_ksplit == 1 ? sms * 8 : wide) : 1;
+    // FMAs: many CTAs of few rows; fragments: one wave, every CTA normalises the step's rows first
+    if (layer >= a.num_layers) return phase != MG_HEAD_LOGITS ? 1 : a.compat_ksplit == 1 && !mg_takes_mma(a.rows, (a.vocab_local + 15) / 16) ? sms * 8 : wide;
     if (a.compat_ksplit == 1) {
+        const int out_rows = a.comm.world == 1 ? a.rows : 1;  // projections with an exchange keep the FMA form (mg_gemv_allreduce)
         switch (phase) {
-        case MG_QKV_A: return capped(one_round((lw.n_qkv_a + 1) / 2, H));
-        case MG_Q_B: { const int g = one_round((lw.n_q_b + 1) / 2, a.Q); return g < a.rows ? a.rows : g; }
-        case MG_OPROJ: return capped(one_round((H + 1) / 2, a.heads_local * a.vdim));
+        case MG_QKV_A: return capped(one_round(a.rows, (lw.n_qkv_a + 15) / 16, (lw.n_qkv_a + 1) / 2, H));
+        case MG_Q_B: { const int g = one_round(a.rows, (lw.n_q_b + 15) / 16, (lw.n_q_b + 1) / 2, a.Q); return g < a.rows ? a.rows : g; }
+        case MG_OPROJ: return capped(one_round(out_rows, (H + 15) / 16, (H + 1) / 2, a.heads_local * a.vdim));
         case MG_MLP_A: {
-            if (lw.dense) return capped(one_round(a.dense_cols, H));
-            const int r = one_round((a.E + 1) / 2, H), sg = one_round(a.shared_cols, H);
+            if (lw.dense) return capped(one_round(a.rows, (a.dense_cols + 7) / 8, a.dense_cols, H));
+            const int r = one_round(a.rows, (a.E + 15) / 16, (a.E + 1) / 2, H), sg = one_round(a.rows, (a.shared_cols + 7) / 8, a.shared_cols, H);
             return capped(r > sg ? r : sg);
         }
         case MG_MLP_B:
-            if (lw.dense) return capped(one_round((H + 1) / 2, a.dense_cols));
+            if (lw.dense) return capped(one_round(out_rows, (H + 15) / 16, (H + 1) / 2, a.dense_cols));
             break;
         default: break;
         }

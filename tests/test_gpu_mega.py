@@ -116,6 +116,24 @@ def test_persistent_kernel_at_eight_lanes_and_glm53_width():
     balanced.close()
 
 
+def test_fused_phases_stream_the_weights_once_for_several_lanes():
+    """The weights are what a step reads, for one lane and for two: the second lane may cost its experts and attention, not the weights again."""
+    g = glm53_geometry().truncated(4)
+    times = []
+    for lanes in (1, 2):
+        runner = _runner(g, None, path="phases", lanes=lanes, capacity=1024, stripe=64, chunk=64, graphs=True)
+        _decode(runner, _prompts(g, (30, 41)[:lanes]), 3)
+        begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        begin.record()
+        for _ in range(20):
+            runner.decode_step()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end))
+        runner.close()
+    assert times[1] < 2.0 * times[0], times  # 1.2 times; 2.8 with a sixteenth of each fragment in use
+
+
 @pytest.mark.parametrize("path", ["phases", "mega"])
 def test_mega_graph_replay_equals_eager_and_frozen_lane_stays_put(path):
     g = small_geometry(4)
