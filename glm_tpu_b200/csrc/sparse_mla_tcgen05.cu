@@ -18,12 +18,16 @@
 // first columns are on their way while the last columns of this block are still being multiplied.  The weights lie where
 // the rotary columns were, which the second product does not need.
 //
-// The running maximum per head is followed only when a score exceeds it by 2^8 (the division at the end removes the difference), so a
-// block costs no reduction over its keys; sums of weights stay per thread until the row ends.  Scores, exponents and sums are fp32, the
-// weights enter the second product as bf16 (as in sparse_mla_rows_kernel, which takes every other shape).
+// Weights are taken relative to the running maximum of their head, block by block, as in sparse_mla_rows_kernel (which takes every other
+// shape): the heaviest weight is then 1 and loses nothing when the weights enter the second product as bf16.  A reference that lags behind by up
+// to 2^8 saves the reduction, but rounds the heaviest weight too (error against 64 bits, 2,048 keys, queries of standard deviation 4: 2.12e-3
+// where 1.73e-3 is reached here and 1.73e-3 by sparse_mla_rows_kernel).  Sums of weights stay per thread until the row ends.  Scores, exponents and sums
+// are fp32.
 //
 // Rows are dealt to one CTA per SM, longest (last) first.  2,048 rows of 2,048 keys on a B200: 5.27 ms with sparse_mla_rows_kernel (111 TFLOP/s),
-// 1.04 ms here (560 TFLOP/s, 4.6 TB/s gathered); 24 rows of 2,048 keys: 170 -> 80 us.
+// 1.04 ms with a
+// lagging reference and a reciprocal (560 TFLOP/s); in a prompt of 4,096 tokens the exact maximum and the division cost 1,017 against 837 us a launch.
+// 24 rows of 2,048 keys: 170 us with sparse_mla_rows_kernel, 80 with a lagging reference.
 //
 // Every wait is bounded; a wait that runs out raises GLMB_STATUS_WAIT_TIMEOUT and the CTA still releases its TMEM.
 #include "attention_core.cuh"
@@ -40,7 +44,6 @@
 #define SM_THREADS 416
 #define SM_SMEM (SM_BOXES * (SM_KBOX + SM_QBOX) + 1024)
 #define SM_LOG2E 1.4426950408889634f
-#define SM_SLACK 8.0f
 
 __device__ __forceinline__ void sm_ld32(uint32_t taddr, float* r) {
     uint32_t v[32];
@@ -67,17 +70,6 @@ __device__ __forceinline__ float sm_exp2(float x) {
     return y;
 }
 __device__ __forceinline__ void sm_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-__device__ __forceinline__ bool sm_barrier_any(bool mine) {  // over the 256 softmax threads
-    uint32_t any;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 q, %1, 0;\n\t"
-        "barrier.cta.red.or.pred p, 1, 256, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(any) : "r"((uint32_t)mine) : "memory");
-    return any != 0;
-}
-
 struct SparseMlaArgs {
     const bf16* kv_cache;
     const int* sel_local;   // [rows, top_k]
@@ -239,45 +231,40 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 float s[SM_HALF];
                 sm_ld32(s_addr, s);
-                bool follow = start == 0;
-                if (start > 0) {
-                    float most = -INFINITY;
+                // the maximum of the warp's keys per head: halves of the heads change sides until lane h has head h
+                float top[SM_HALF];
 #pragma unroll
-                    for (int h = 0; h < SM_HALF; h += 4) {
-                        const float4 m = *reinterpret_cast<const float4*>(ref + h);
-                        most = fmaxf(most, fmaxf(fmaxf(fmaf(s[h], scale2, -m.x), fmaf(s[h + 1], scale2, -m.y)),
-                                                 fmaxf(fmaf(s[h + 2], scale2, -m.z), fmaf(s[h + 3], scale2, -m.w))));
-                    }
-                    follow = sm_barrier_any(live && most > SM_SLACK);
-                }
-                if (follow) {  // all eight warps: the maximum of the block per head
-                    float top = -INFINITY;
+                for (int h = 0; h < SM_HALF; ++h) top[h] = live ? s[h] * scale2 : -INFINITY;
 #pragma unroll
-                    for (int h = 0; h < SM_HALF; ++h) {
-                        const float m = warp_max(live ? s[h] * scale2 : -INFINITY);
-                        if (lane == h) top = m;
-                    }
-                    top_s[warp][lane] = top;
-                    sm_barrier();
-                    const float (*tops)[SM_HALF] = top_s + half * 4;
-                    const float next = fmaxf(run, fmaxf(fmaxf(tops[0][lane], tops[1][lane]), fmaxf(tops[2][lane], tops[3][lane])));
-                    fix[lane] = next == -INFINITY ? 1.f : sm_exp2(run - next);
-                    ref[lane] = next == -INFINITY ? 0.f : next;
-                    run = next;
-                    __syncwarp();
-                    if (start > 0) {  // the products of the block before are complete: the scores of this one follow them
+                for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                        for (int h = 0; h < SM_HALF; ++h) l[h] *= fix[h];
-#pragma unroll 1
-                        for (int c = 0; c < SM_L / 2; c += 64) {
-                            float o[32];
-                            sm_ld32(o_addr + c, o);
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) o[e] *= fix[e];
-                            sm_st32(o_addr + c, o);
+                    for (int h = 0; h < 16; ++h)
+                        if (h < o) {
+                            const bool up = lane & o;
+                            const float keep = up ? top[h + o] : top[h], send = up ? top[h] : top[h + o];
+                            top[h] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, o));
                         }
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                top_s[warp][lane] = top[0];
+                sm_barrier();  // (nobody writes the next block's before all have given up this block's weights)
+                const float (*tops)[SM_HALF] = top_s + half * 4;
+                const float next = fmaxf(run, fmaxf(fmaxf(tops[0][lane], tops[1][lane]), fmaxf(tops[2][lane], tops[3][lane])));
+                const float factor = next == -INFINITY ? 1.f : sm_exp2(run - next);
+                fix[lane] = factor;
+                ref[lane] = next == -INFINITY ? 0.f : next;
+                run = next;
+                __syncwarp();
+                if (__any_sync(0xffffffffu, factor != 1.f) && start > 0) {  // the products of the block before are complete: the scores of this one follow them
+#pragma unroll
+                    for (int h = 0; h < SM_HALF; ++h) l[h] *= fix[h];
+#pragma unroll 1
+                    for (int c = 0; c < SM_L / 2; c += 64) {
+                        float o[32];
+                        sm_ld32(o_addr + c, o);
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) o[e] *= fix[e];
+                        sm_st32(o_addr + c, o);
                     }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 }
 #pragma unroll
                 for (int c = 0; c < SM_HALF; c += 8) {
@@ -312,7 +299,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
             sum_s[warp][lane] = l[0];
             sm_barrier();
             const float (*sums)[SM_HALF] = sum_s + half * 4;
-            fix[lane] = 1.f / ((sums[0][lane] + sums[1][lane]) + (sums[2][lane] + sums[3][lane]));
+            fix[lane] = (sums[0][lane] + sums[1][lane]) + (sums[2][lane] + sums[3][lane]);
             __syncwarp();
             if (ok) ok = mbar_wait_warp(o_done + 3, (n - 1) & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -323,7 +310,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
                 const int at = c * 128 + (warp & 3) * 32 + (lane & ~1);
 #pragma unroll
                 for (int e = 0; e < 32; e += 2) {  // neighbours swap, so that each stores two columns of one head
-                    const float x = o[e] * fix[e], y = o[e + 1] * fix[e + 1];
+                    const float x = o[e] / fix[e], y = o[e + 1] / fix[e + 1];  // the contract divides (no reciprocal)
                     const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? x : y, 1);
                     if (ok) *reinterpret_cast<uint32_t*>(out + (e + (lane & 1)) * SM_L + at) = (lane & 1) ? pack_bf16(got, y) : pack_bf16(x, got);
                 }

@@ -79,3 +79,26 @@ def test_growing_scores_follow_the_maximum_and_bad_rows_are_reported(native_lib)
     q[0, 3, 7] = float("inf")
     _, status = _run(native_lib, q, cache, sel, cnt, lane, count, scale)
     assert status & native_lib.STATUS_NONFINITE
+
+
+@pytest.mark.parametrize("count,spread", [(200, 1.0), (2048, 0.3), (2048, 1.0), (2048, 4.0), (2048, 12.0)])
+def test_rounding_the_weights_costs_what_it_must(native_lib, count, spread):
+    """The error is that of weights rounded to bf16 beside the heaviest, which is 1, and of a rounded result; however sharp the softmax is."""
+    rows, cap = 24, 4096
+    q, cache, sel, cnt, lane = _case([count] * rows, count, cap, seed=3, spread=spread)
+    scale = W**-0.5
+    out, status = _run(native_lib, q, cache, sel, cnt, lane, count, scale)
+    assert status == 0
+    got, best, size = 0.0, 0.0, 0.0
+    for r in range(rows):
+        k = cache[1, 1, sel[r, :count].long()].double()
+        score = q[r].double() @ k.T * scale
+        weight = torch.exp(score - score.max(dim=1, keepdim=True).values)
+        total = weight.sum(dim=1, keepdim=True)
+        want = weight @ k[:, :L] / total
+        rounded = (weight.to(torch.bfloat16).double() @ k[:, :L] / total).to(torch.bfloat16).double()
+        got += float((out[r].double() - want).square().sum())
+        best += float((rounded - want).square().sum())
+        size += float(want.square().sum())
+    # the maximum is that of the blocks so far: a few weights of early blocks are rounded beside a smaller one, by the same 2^-9 at most
+    assert got**0.5 <= 1.06 * best**0.5, (got / size, best / size)
