@@ -13,6 +13,8 @@
 //   warps 2-5   epilogue of this CTA's 128 rows; the TMEM holds two accumulators, so it runs while the next tile is multiplied
 //
 // Tiles are walked by one pair per two SMs, in groups of eight row tiles by all column tiles (operand tiles shared in L2).
+// The activation of the gated form is glu_activation, as in a launch of its own: the same bits (a quotient and a tanh without branches save nothing
+// measurable: the epilogue runs beside the next tile's products).
 // Bound by the tensor core (and the power it may draw).  Measured on a B200, single SMs -> pairs: [8192 x 8192], K 8192: 809 -> 717 us (1,534
 // TFLOP/s); [4096 x 28672], K 4096: 718 -> 614; gated [4096 x 2 x 14336], K 4096, with its activation: 797 -> 609.
 #pragma once
@@ -51,14 +53,6 @@ __device__ __forceinline__ void gp_commit(uint64_t* bar) {  // arrives at this b
 }
 __device__ __forceinline__ void gp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// f(z) of a gated pair without a branch: one warp per scheduler runs the epilogue, so that the slow paths of an IEEE division and of tanh
-// would serialise its elements.  0.5 z (1 + tanh(u)) is z / (1 + exp(-2 u)); the quotient is within a few units in the last place of fp32,
-// 2^-13 of the rounding to bf16 that follows.
-__device__ __forceinline__ float gp_activation(int kind, float z) {
-    const float y = kind == GLU_SILU ? z : 1.5957691216057308f * (z + 0.044715f * z * z * z);  // 2 sqrt(2 / pi)
-    return z * __fdividef(1.f, 1.f + expf(-y));
 }
 
 struct GemmPairArgs {
@@ -184,7 +178,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         float v[2];
 #pragma unroll
                         for (int q = 0; q < 2; ++q)
-                            v[q] = gp_activation(p.glu, bf16_round(__uint_as_float(g[2 * e + q]))) * bf16_round(__uint_as_float(u[2 * e + q]));
+                            v[q] = glu_activation(p.glu, bf16_round(__uint_as_float(g[2 * e + q]))) * bf16_round(__uint_as_float(u[2 * e + q]));
                         o[e] = pack_bf16(v[0], v[1]);
                     }
                     if (row < p.rows)

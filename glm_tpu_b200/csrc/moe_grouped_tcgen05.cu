@@ -22,8 +22,8 @@
 //
 // What bounds it: the FP8 bytes, which cross HBM once (5.2 - 5.7 TB/s up to 777 rows), and with many routes the epilogue of tiles of more than
 // 64 routes, which have one accumulator.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 1,061 + 554 us
-// (routes as the M in tiles of 128: 1,931 + 1,065; decoded weights through shared memory: 1,680 + 856); 2,048 rows 1,593 + 1,007 (2,377 +
-// 1,302; 1,891 + 1,034), and 1,413 + 799 since the epilogue has no division and no per-column loads of the route list.
+// (a kernel with the routes as the M and decoded weights in shared memory: 1,931 + 1,065); 2,048 rows 1,413 + 799 us (2,377 + 1,302) with an approximate
+// quotient in the activation, and 6 % more (1,247 against 1,174 us a launch in a prompt of 4,096 tokens) with the exact one, whose results are those of the other forms of this projection bit for bit.
 // Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores and
 // still frees its TMEM.
 //
@@ -267,7 +267,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             const float gv = bf16_round(__uint_as_float(g[e + q])), uv = bf16_round(__uint_as_float(u[e + q]));
-                            v[q] = gv * __fdividef(1.f, 1.f + expf(-gv)) * uv;  // no branch: an IEEE division would serialise the elements
+                            v[q] = gv * sigmoidf_precise(gv) * uv;
                         }
                         const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[0] : v[1], 1);
                         const int r = r0 + e + (lane & 1);

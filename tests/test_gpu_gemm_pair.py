@@ -56,3 +56,35 @@ def test_gated_form_equals_two_launches(native_lib, rows, N, K, kind):
     floor = 2.0**-23 * (both[:, :N].float() * both[:, N:].float()).abs()
     assert ((got - want).abs() <= 2**-7 * want.abs() + floor).all() and float(((got - want).abs() > floor).float().mean()) < 0.01
     assert wide[1][:, :8].isnan().all() and wide[1][:, N + 8 :].isnan().all()
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_gated_form_over_several_tiles_per_pair(native_lib, kind):
+    """11 x 23 tiles for 74 pairs of SMs, ragged rows, columns and K: accumulators handed back while the next tile is multiplied; the two-launch form's bits."""
+    rows, N, K = 2600, 2824, 136
+    a, b = _operands(rows, 2 * N, K, seed=7)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    both = torch.empty(rows, 2 * N, dtype=torch.bfloat16, device="cuda")
+    native_lib.gemm_bf16_tc(a, b, both, status=status)
+    two, one = (torch.full((rows + 1, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    native_lib.glu_rows(both[:, :N], both[:, N:], two[:rows], kind)
+    native_lib.gemm_bf16_gated(a, b[:N], b[N:], one[:rows], kind, status=status)
+    torch.cuda.synchronize()
+    assert int(status) == 0 and one[rows].isnan().all()
+    assert torch.equal(one[:rows], two[:rows])
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_gated_form_has_the_bits_of_two_launches_far_from_zero(native_lib, kind):
+    """Gates from -100 to 100, where the activation underflows or saturates."""
+    rows, N, K = 300, 264, 64
+    a, b = _operands(rows, 2 * N, K, seed=9)
+    b = (b.float() * 20).to(torch.bfloat16)
+    both = torch.empty(rows, 2 * N, dtype=torch.bfloat16, device="cuda")
+    native_lib.gemm_bf16_tc(a, b, both)
+    assert float(both[:, :N].min()) < -100 and float(both[:, :N].max()) > 100
+    two, one = (torch.empty(rows, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    native_lib.glu_rows(both[:, :N], both[:, N:], two, kind)
+    native_lib.gemm_bf16_gated(a, b[:N], b[N:], one, kind)
+    torch.cuda.synchronize()
+    assert torch.equal(one, two)

@@ -147,3 +147,69 @@ def test_swiglu_rows_matches_the_elementwise_expression(native_lib):
     assert float((out != ref).float().mean()) < 1e-3  # at most a last-place difference of the exponential here and there
     inplace = gate.clone()
     assert n.swiglu_rows(inplace, up, inplace) is inplace and torch.equal(inplace, out)
+
+
+def _codes(gen, *shape):
+    return (torch.randn(*shape, device=DEV, generator=gen) * 64).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+
+
+def _decoded(codes, scale):
+    """``bf16(f32(e4m3) * scale)`` of one expert, in 64 bits."""
+    n, k = codes.shape
+    return (codes.view(torch.float8_e4m3fn).float() * scale.repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)[:, :k]).bfloat16().double()
+
+
+# many items per CTA, narrow tiles after wide ones and the reverse, every number of routes around the steps of 16, 64 and 128; then sizes that
+# end inside a block of 128 output columns, 256 output columns and 128 columns of K
+@pytest.mark.parametrize("H,I,O,counts", [
+    (2560, 2048, 2560, [1, 128, 16, 300, 64, 17, 65, 0, 129, 15, 127, 2] * 4),
+    (144, 136, 392, [5, 0, 70, 130]),
+    (400, 264, 136, [33, 129, 1]),
+])
+def test_grouped_kernel_over_many_tiles(native_lib, H, I, O, counts):  # noqa: E741
+    n, el = native_lib, len(counts)
+    gen = torch.Generator(device=DEV).manual_seed(H)
+    local = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)] + [torch.full((50,), el)])  # the last fifty: experts of another GPU
+    local = local[torch.randperm(local.numel(), generator=torch.Generator().manual_seed(1))]
+    tiles, n_tiles, perm = (t.to(DEV) for t in _tiles(local, el))
+    P, here = local.numel(), sum(counts)
+    x = (torch.randn(P, H, device=DEV, generator=gen) * 0.5).bfloat16()
+    weight = torch.rand(P, device=DEV, generator=gen) + 0.1
+    wg, wu = _codes(gen, el, I, H), _codes(gen, el, I, H)
+    sg, su = ((torch.rand(el, -(-I // 128), -(-H // 128), device=DEV, generator=gen) + 0.5) * (2 * H**-0.5 / 64) for _ in range(2))
+    xs = torch.full((P, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+    n.gather_rows(x, perm, 1, xs)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    acts = [torch.full((P, I), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for out in acts:
+        n.moe_grouped_fp8w(xs, wg, wu, sg, su, tiles, n_tiles, 0, out, status=status)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    assert torch.equal(acts[0][:here], acts[1][:here]) and acts[0][here:].isnan().all()
+    # the second half on activations of its own, whose K is a multiple of 16
+    K = (I + 15) // 16 * 16
+    mid = (torch.randn(P, K, device=DEV, generator=gen) * 0.5).bfloat16()
+    wd, sd = _codes(gen, el, O, K), (torch.rand(el, -(-O // 128), -(-K // 128), device=DEV, generator=gen) + 0.5) * (K**-0.5 / 64)
+    dws = [torch.full((P, O), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for out in dws:
+        n.moe_grouped_fp8w(mid, wd, None, sd, None, tiles, n_tiles, 1, out, perm=perm, route_weight=weight, status=status)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    foreign = (local >= el).nonzero().flatten().to(DEV)
+    assert dws[0][foreign].isnan().all() and not dws[0][perm[:here].long()].isnan().any()
+    assert torch.equal(dws[0].nan_to_num(7.0), dws[1].nan_to_num(7.0))
+    start = 0
+    for e, c in enumerate(counts):
+        rows, routes = xs[start : start + c].double(), perm[start : start + c].long()
+        if c:
+            g, u = (rows @ _decoded(w[e], s[e]).T for w, s in ((wg, sg), (wu, su)))
+            off_g, off_u = ((H / 16 + 16) * 2.0**-24 * (rows.abs() @ _decoded(w[e], s[e]).abs().T) for w, s in ((wg, sg), (wu, su)))  # fp32 sums, truncated
+            gr, ur = g.bfloat16().double(), u.bfloat16().double()
+            want = gr * torch.sigmoid(gr) * ur
+            # a product may land on the neighbouring bf16 (2^-7 for both), the gate's slope is at most 1.1, and the result is rounded once more
+            bound = 2**-8 * want.abs() + 1.1 * (2**-8 * gr.abs() + off_g) * ur.abs() + (2**-8 * ur.abs() + off_u) * gr.abs()
+            assert ((acts[0][start : start + c].double() - want).abs() <= 1.01 * bound).all(), (e, c)
+            d = mid[start : start + c].double() @ _decoded(wd[e], sd[e]).T
+            want = d * weight[routes].bfloat16().double()[:, None]
+            assert ((dws[0][routes].double() - want).abs() <= 2**-7 * want.abs() + 2e-5).all(), (e, c)  # rounded twice; fp32 sums of K products of size K^-1/2
+        start += c
