@@ -161,7 +161,7 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     __syncwarp();
                 }
             }
-            if (!ok) { fail = 1; break; }
+            if (!ok || __any_sync(0xffffffffu, fail)) { fail = 1; break; }
             if (elect_one()) {
                 if (j >= 0) umma_commit(v_empty + j % FA_STAGES);            // the blocks may be replaced once these products have read them
                 if (j + 1 < blocks) umma_commit(k_empty + (j + 1) % FA_STAGES);

@@ -247,7 +247,7 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     if (warp == 0) {
         uint32_t g = 0;  // k-blocks issued so far, across tiles
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int t = blockIdx.x; t < total && ok && !__any_sync(0xffffffffu, *fail_slot); t += gridDim.x) {
             int m, n;
             const int head = t / per_problem;
             t2_tile(t % per_problem, m_tiles, n_blocks, m, n);
@@ -273,7 +273,7 @@ gemm_bf16_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, T2_BN) | (MN ? 1u << 16 : 0u);  // bit 16: B is MN-major
         uint32_t g = 0, i = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
+        for (int t = blockIdx.x; t < total && !__any_sync(0xffffffffu, *fail_slot); t += gridDim.x, ++i) {
             const uint32_t acc = i & 1, use = i >> 1;
             if (use > 0 && !mbar_wait_warp(acc_empty + acc, (use - 1) & 1)) { *fail_slot = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
