@@ -251,11 +251,12 @@ chunk_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 for (int c = 0; c < a.vdimp; c += 16) {
                     uint32_t o[16];
                     tmem_ld16(o_addr + c, o);
-                    if (row >= range[t].rows) continue;
                     uint32_t w[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) w[i] = pack_bf16(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
-                    if (vec && c + 16 <= a.vdim) {
+                    if (row >= range[t].rows) {
+                        // a row past the tile's end
+                    } else if (vec && c + 16 <= a.vdim) {
                         *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
                         *reinterpret_cast<uint4*>(dst + c + 8) = make_uint4(w[4], w[5], w[6], w[7]);
                     } else {

@@ -191,15 +191,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 for (int cb = 0; cb < cols; cb += 32) {
                     uint32_t v[32];
                     tmem_ld32(d + cb, v);
-                    if (row >= p.rows) continue;
-                    if (p.out == GP_OUT_F32) {
+                    if (row < p.rows && p.out == GP_OUT_F32) {
                         float* dst = reinterpret_cast<float*>(p.c) + (int64_t)row * p.ldc + n0 + cb;
 #pragma unroll
                         for (int e = 0; e < 32; e += 4)
                             if (n0 + cb + e < p.N)
                                 *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]),
                                                                                   __uint_as_float(v[e + 3]));
-                    } else {
+                    } else if (row < p.rows) {
                         bf16* dst = reinterpret_cast<bf16*>(p.c) + (int64_t)row * p.ldc + n0 + cb;
 #pragma unroll
                         for (int e = 0; e < 32; e += 8)
