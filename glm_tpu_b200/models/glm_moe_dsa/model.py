@@ -208,8 +208,10 @@ class GlmMoeDsaModel:
         # the one-launch expert sort takes up to 256 resident experts and contiguous ids; other shapes use the library-op sort
         # (`_route_tiles128`), and tests set this attribute to compare the two on shapes both take
         self.route_sort_kernel = True
-        self.few_routes_gemv = True  # prefill chunks of up to 256 rows with few routes per expert on average: GEMV kernels on 8-route tiles (tests compare)
-        self.few_routes_limit = int(os.environ.get("GLM_B200_FEW_ROUTES", "12"))  # mean routes per expert up to which that path is taken
+        self.few_routes_gemv = True  # prefill chunks with few routes per expert on average: GEMV kernels on 8-route tiles
+        # mean routes per expert up to which that path is taken: a limit of the user's holds for every chunk, the default for those of up to 256 rows
+        self.few_routes_limit = int(os.environ.get("GLM_B200_FEW_ROUTES", "12"))
+        self.few_routes_rows = None if "GLM_B200_FEW_ROUTES" in os.environ else 256
         self.merge_vproj = os.environ.get("GLM_B200_MERGE_VPROJ", "1") != "0"  # decode: chunk merge + value projection in one launch
         self.prefill_rows_attention = os.environ.get("GLM_B200_PREFILL_ATTENTION", "rows") != "split"
         # Prefill projections whose K is split over the GPUs use the GEMM with the all-reduce in its epilogue (about 1.2x the
@@ -303,7 +305,7 @@ class GlmMoeDsaModel:
     def _heads_gemm(self, rows: int, kv_b: torch.Tensor) -> bool:
         """Whether the per-head products of a prefill chunk (absorbed query, value projection) take the batched tcgen05 GEMM, which reads
         queries and writes results where they lie; the library's form copies both (2,048 rows of 64 heads: 157 us each, 120 of them copies, against
-        71 and 47 us).  Few rows keep the library's form and their recorded launch program."""
+        71 and 47 us).  Chunks of up to 256 rows, where the two were not compared, keep the library's form: their launch program is recorded with it."""
         g = self.g
         return (rows > 256 and g.qk_nope_head_dim % 64 == 0 and g.kv_lora_rank % 64 == 0 and g.v_head_dim % 8 == 0 and g.kv_row_width % 8 == 0
                 and kv_b.is_contiguous() and kv_b.data_ptr() % 16 == 0)
@@ -591,11 +593,12 @@ class GlmMoeDsaModel:
             self.trace.setdefault("topk_ids", {})[layer] = ws.topk_ids[:rows].clone()
             self.trace.setdefault("topk_w", {})[layer] = ws.topk_w[:rows].clone()
         sort_kernel = self.route_sort_kernel and el <= 256 and ws.topk_ids[:rows].is_contiguous()
-        # A short chunk with few routes per expert (200 rows x 8 routes over 256 experts are ~6 each) runs the GEMV kernels on 8-route tiles:
-        # the launch program that chunks of up to 256 rows are recorded with.  Longer ones take the grouped GEMM, which reads an expert once
-        # however many tiles of eight its routes fill.  Measured, gate/up + down of a layer of 256 experts: 300 rows 1,867 + 1,233 (GEMV) against
-        # 967 + 504 us, 380 rows 2,166 + 1,436 against 975 + 507; one rank's shard of eight, 300 rows: 231 + 187 against 130 + 98.
-        few_per_expert = self.few_routes_gemv and sort_kernel and rows <= 256 and rows * tk < self.few_routes_limit * E
+        # The grouped GEMM reads an expert once however many routes it has and is the faster form at every count measured, gate/up + down of a
+        # layer of 256 experts: 200 rows 2,536 us (GEMV kernels on 8-route tiles) against 1,460, 300 rows 1,867 + 1,233 against 967 + 504, 380 rows
+        # 2,166 + 1,436 against 975 + 507; one rank's shard of eight, 300 rows: 231 + 187 against 130 + 98.  Chunks of up to 256 rows keep
+        # the GEMV kernels for one reason only: their launch program is recorded with them, and a changed one is accepted in a step of its own.
+        short = self.few_routes_rows is None or rows <= self.few_routes_rows
+        few_per_expert = self.few_routes_gemv and sort_kernel and short and rows * tk < self.few_routes_limit * E
         if not decode and not few_per_expert and rows * tk >= 128 and H % 16 == 0 and I % 16 == 0:
             # many rows: expert-sorted routes through the tcgen05 grouped GEMM (FP8 decoded inside the kernel)
             if sort_kernel:
