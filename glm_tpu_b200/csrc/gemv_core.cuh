@@ -79,7 +79,8 @@ __device__ __forceinline__ void warp_reduce_all(float (&acc)[NPW][R]) {
 }
 
 // ---------------------------------------------------------------------------------------------------
-// 16 weight rows as the M and one to eight activation rows as the N of mma.sync m16n8k16 (bf16 products, fp32 sums).  With R rows the
+// 16 weight rows as the M and one to eight activation rows as the N of mma.sync m16n8k16 (bf16 products, fp32 sums).  A row's bits depend neither on
+// how many others there are (from two rows on) nor on what they hold; a row alone takes the FMA kernel, which adds in another order.  With R rows the
 // FMA loop above issues R + 2 instructions per weight and is bound by issue from four rows on; here a weight costs a sixteenth of an
 // instruction whatever R is, and nothing is shuffled at the end.  Measured on a B200, [6144 x 16384]: 2 rows 49.8 -> 32.2 us, 4 rows
 // 58.0 -> 32.6, 8 rows 85.5 -> 32.9 (6.1 TB/s); [131072 x 4096]: 193 -> 154, 218 -> 158, 397 -> 163.
