@@ -22,8 +22,9 @@
 //
 // What bounds it: the FP8 bytes, which cross HBM once (5.2 - 5.7 TB/s up to 777 rows), and with many routes the epilogue of tiles of more than
 // 64 routes, which have one accumulator.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 1,061 + 554 us
-// (a kernel with the routes as the M and decoded weights in shared memory: 1,931 + 1,065); 2,048 rows 1,413 + 799 us (2,377 + 1,302) with an approximate
-// quotient in the activation, and 6 % more (1,247 against 1,174 us a launch in a prompt of 4,096 tokens) with the exact one, whose results are those of the other forms of this projection bit for bit.
+// (a kernel with the routes as the M and decoded weights in shared memory: 1,931 + 1,065); 2,048 rows 1,413 + 799 us (2,377 + 1,302) with an
+// approximate quotient in the activation.  The exact one, whose results are those of the other forms of this projection bit for bit, costs 6 % (1,247
+// against 1,174 us a launch, both directions, in a prompt of 4,096 tokens).
 // Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores and
 // still frees its TMEM.
 //

@@ -20,14 +20,13 @@
 //
 // Weights are taken relative to the running maximum of their head, block by block, as in sparse_mla_rows_kernel (which takes every other
 // shape): the heaviest weight is then 1 and loses nothing when the weights enter the second product as bf16.  A reference that lags behind by up
-// to 2^8 saves the reduction, but rounds the heaviest weight too (error against 64 bits, 2,048 keys, queries of standard deviation 4: 2.12e-3
-// where 1.73e-3 is reached here and 1.73e-3 by sparse_mla_rows_kernel).  Sums of weights stay per thread until the row ends.  Scores, exponents and sums
-// are fp32.
+// to 2^8 saves the reduction, but rounds the heaviest weight too: against 64 bits, 2,048 keys, queries of standard deviation 4, the result is
+// then 2.12e-3 off, here and by sparse_mla_rows_kernel 1.73e-3.  Sums of weights stay per thread until the row ends.  Scores, exponents and
+// sums are fp32.
 //
-// Rows are dealt to one CTA per SM, longest (last) first.  2,048 rows of 2,048 keys on a B200: 5.27 ms with sparse_mla_rows_kernel (111 TFLOP/s),
-// 1.04 ms with a
-// lagging reference and a reciprocal (560 TFLOP/s); in a prompt of 4,096 tokens the exact maximum and the division cost 1,017 against 837 us a launch.
-// 24 rows of 2,048 keys: 170 us with sparse_mla_rows_kernel, 80 with a lagging reference.
+// Rows are dealt to one CTA per SM, longest (last) first.  2,048 rows of 2,048 keys on a B200: 5.27 ms with sparse_mla_rows_kernel (111 TFLOP/s), 1.04
+// ms here with a lagging reference and a reciprocal (560 TFLOP/s); the exact maximum and the division cost 1,017 against 837 us a launch in a
+// prompt of 4,096 tokens.
 //
 // Every wait is bounded; a wait that runs out raises GLMB_STATUS_WAIT_TIMEOUT and the CTA still releases its TMEM.
 #include "attention_core.cuh"
