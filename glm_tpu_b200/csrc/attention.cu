@@ -375,7 +375,7 @@ GLMB_API int glmb_sparse_mla_rows(const void* q_full, const void* kv_cache, cons
                                   uint32_t* status, void* stream) {
     if (((L + rd) & 15) || rows < 1) return 1;
     cudaStream_t st = (cudaStream_t)stream;
-    // the flagship's head shape at any number of rows (24 rows of 2,048 keys: 170 -> 80 us, 200 of 200: 84 -> 30; a fifth more since it follows its maximum exactly)
+    // the flagship's head shape at any number of rows (24 rows of 2,048 keys: 170 -> 97 us, 200 of 200: 84 -> 36)
     if (sparse_mla_tc_takes(q_full, kv_cache, o_lat, H, L, rd))
         return launch_sparse_mla_tc(q_full, kv_cache, sel_local, sel_counts, row_lane, rows, layer, layers, local_cap, top_k, scale, o_lat, status, st);
 #define ARGS q_full, kv_cache, sel_local, sel_counts, row_lane, rows, H, rd, layer, layers, local_cap, top_k, scale, o_lat, status, st
