@@ -108,22 +108,37 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // 1: launch with the programmatic-serialization attribute (default); 0: plain stream order.
 extern int g_glmb_pdl_enabled;
 
+// `carveout`: percent of an SM's L1 that is to be shared memory (-1: whatever the SM has, as long as the CTA fits).
 template <typename... KArgs, typename... Args>
-static inline cudaError_t glmb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                      Args&&... args) {
+static inline cudaError_t glmb_launch_carved(int carveout, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                             Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = g_glmb_pdl_enabled ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (carveout >= 0) {
+        attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[1].val.sharedMemCarveout = carveout;
+        cfg.numAttrs = 2;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
-#define GLMB_LAUNCH(kernel, grid, block, smem, stream, ...) (void)glmb_launch(kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__)
+#define GLMB_LAUNCH(kernel, grid, block, smem, stream, ...) (void)glmb_launch_carved(-1, kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__)
+// For kernels whose loads in flight live in the L1 (weights streamed into registers by many warps, activations read again and again) and that have a few
+// KB of shared memory.  Chained by programmatic dependent launch an SM is never idle, so without a preference it keeps the split that the last kernel with a
+// large ring (attention, indexer: up to 200 KB) needed, and what is left of the L1, 28 KB, bounds the bytes in flight.  15 % is 32 KB of shared memory,
+// three CTAs.  Measured in captured decode steps on a B200: eight chats of the medium Namizen 1,573 -> 905 us a step ([4096 x 18432] 79 -> 30, head
+// [131072 x 4096] 340 -> 175), four of GLM at 5,000 1,875 -> 1,729, eight of the routed Zikevik 1,720 -> 1,557; with 8, 25 and 50 % 974, 971, 970 us for the
+// first.  Not for projections of one row (FMA): 25 % 1,058 -> 1,095 us in GLM, 15 % no change.
+#define GLMB_L1_CARVEOUT 15
+#define GLMB_LAUNCH_L1(kernel, grid, block, smem, stream, ...) \
+    (void)glmb_launch_carved(GLMB_L1_CARVEOUT, kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__)
 
 // A once-per-device latch for settings that belong to a device, not to the process (cudaFuncSetAttribute: the opt-in to large
 // dynamic shared memory has to be repeated on every GPU a process drives).  `pending()` names the current device if the setting

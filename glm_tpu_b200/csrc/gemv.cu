@@ -296,7 +296,7 @@ GLMB_API int glmb_skinny_bf16(const void* x, int64_t xs, int rows, const void* w
     const int groups = ceil_div(N, 16);
     if (rows > 1 && skinny_mma_takes(groups) && batch == 1 && !(mode == SK_OUT_ALLREDUCE_BF16 && c.world > 1)) {
 #define CALL(D)                                                                                                                            \
-    GLMB_LAUNCH(skinny_mma_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)w, ws, N, K, out, os, mode, \
+    GLMB_LAUNCH_L1(skinny_mma_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)w, ws, N, K, out, os, mode, \
                 c.status, channel)
         if (skinny_mma_depth(groups, K) == 4) CALL(4);
         else CALL(2);
@@ -325,7 +325,7 @@ GLMB_API int glmb_skinny_bf16_swiglu(const void* x, int64_t xs, int rows, const 
     const int groups = ceil_div(N, 8);
     if (rows > 1 && skinny_mma_takes(groups)) {
 #define CALL(D)                                                                                                                                   \
-    GLMB_LAUNCH(skinny_mma_swiglu_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)wg, (const bf16*)wu, ws, \
+    GLMB_LAUNCH_L1(skinny_mma_swiglu_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)wg, (const bf16*)wu, ws, \
                 N, K, (bf16*)act, as)
         if (skinny_mma_depth(groups, K) == 4) CALL(4);
         else CALL(2);

@@ -222,7 +222,7 @@ GLMB_API int glmb_expert_glu(const void* x, int64_t xs, int rows, int top, const
     if (rows < 1 || top < 1 || (int64_t)rows * top > 65535 || E < 1 || F < 1 || (K & 7) || K < 8 || (xs & 7) || (kind != GLU_SILU && kind != GLU_GELU_TANH)) return 1;
     const dim3 grid(ceil_div(F, MR_WARPS), rows * top);
     if (!is_f32 && rows <= MR_ROWS && rows * top <= MR_ROUTES && !(F & 7))
-        GLMB_LAUNCH(expert_glu_mma_kernel, grid, MR_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, top, ids, weights, (const bf16*)gate_up, E, F, K,
+        GLMB_LAUNCH_L1(expert_glu_mma_kernel, grid, MR_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, top, ids, weights, (const bf16*)gate_up, E, F, K,
                     kind, (bf16*)act, status);
     else if (is_f32)
         GLMB_LAUNCH(expert_glu_kernel<float>, grid, MR_THREADS, 0, (cudaStream_t)stream, (const float*)x, xs, top, ids, weights, (const float*)gate_up, E, F, K, kind,
@@ -239,7 +239,7 @@ GLMB_API int glmb_expert_down(const void* act, int rows, int top, const int* ids
     if (rows < 1 || rows > 65535 || top < 1 || E < 1 || N < 1 || (F & 7) || F < 8) return 1;
     const dim3 grid(ceil_div(N, MR_WARPS), rows);
     if (!is_f32 && rows <= MR_ROWS && rows * top <= MR_ROUTES)
-        GLMB_LAUNCH(expert_down_mma_kernel, ceil_div(N, 16), MR_THREADS, rows * top * 32 * sizeof(float), (cudaStream_t)stream, (const bf16*)act, rows, top, ids,
+        GLMB_LAUNCH_L1(expert_down_mma_kernel, ceil_div(N, 16), MR_THREADS, rows * top * 32 * sizeof(float), (cudaStream_t)stream, (const bf16*)act, rows, top, ids,
                     (const bf16*)down, E, N, F, out, os);
     else if (is_f32)
         GLMB_LAUNCH(expert_down_kernel<float>, grid, MR_THREADS, 0, (cudaStream_t)stream, (const float*)act, top, ids, (const float*)down, E, N, F, out, os);

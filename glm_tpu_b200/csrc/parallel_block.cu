@@ -246,7 +246,7 @@ GLMB_API int glmb_dual_proj(const void* x1, const void* x2, int64_t xs, int rows
     }
     const int proj_blocks = ceil_div(N, 16), grid = proj_blocks + ceil_div(F, 8);
 #define CALL(D)                                                                                                                                      \
-    GLMB_LAUNCH(dual_proj_kernel<D>, grid, DP_THREADS, 0, (cudaStream_t)stream, (const bf16*)x1, (const bf16*)x2, xs, rows, K, (const bf16*)w, N, (bf16*)out, \
+    GLMB_LAUNCH_L1(dual_proj_kernel<D>, grid, DP_THREADS, 0, (cudaStream_t)stream, (const bf16*)x1, (const bf16*)x2, xs, rows, K, (const bf16*)w, N, (bf16*)out, \
                 os, (const bf16*)wg, (const bf16*)wu, F, (bf16*)act, as, kind, proj_blocks)
     if (skinny_mma_depth(grid, K) == 4) CALL(4);
     else CALL(2);
