@@ -235,6 +235,11 @@ int glmb_launch_moe_gateup_mma(const void* x, int64_t xs, int top_k, const int* 
 int glmb_launch_moe_down_mma(const void* act, const float* route_weight, const int* tile_expert, const int* tile_routes, const int* n_tiles,
                              int tiles, int rt, const void* wd, const float* sd, int expert_base, int experts_local, int I, int H, void* dw,
                              cudaStream_t stream);
+// Tiles of eight routes on tcgen05 (moe_grouped_tcgen05.cu).
+bool moe_tiles8_takes(const void* x, int64_t x_stride, const void* w0, const void* w1, const void* out, const int* tile_routes, int tiles, int experts, int N, int K);
+int launch_moe_tiles8(const void* x, int64_t x_stride, int divisor, const int* tile_expert, const int* tile_routes, const int* n_tiles, int tiles,
+                      const void* w0, const void* w1, const float* s0, const float* s1, int expert_base, int experts_local, int N, int K, int mode,
+                      const float* route_weight, void* out, cudaStream_t stream);
 static int g_moe_mma = 1;
 // The fp32-FMA kernels below serve the shapes the mma.sync kernels refuse (hidden size not a multiple of 64, intermediate not a
 // multiple of 16, unaligned rows: fixtures).  The switch exists so that the tests can run BOTH families on shapes both take
@@ -246,6 +251,9 @@ GLMB_API int glmb_moe_gateup_fp8(const void* x, int64_t xs, int top_k, const int
                                  const int* n_tiles, int tiles, int rt, const void* wg, const void* wu, const float* sg,
                                  const float* su, int expert_base, int experts_local, int I, int H, void* act, void* stream) {
     if ((H & 15) || tiles < 1) return 1;
+    if (g_moe_mma && rt == 8 && top_k > 0 && moe_tiles8_takes(x, xs, wg, wu, act, tile_routes, tiles, experts_local, I, H))
+        return launch_moe_tiles8(x, xs, top_k, tile_expert, tile_routes, n_tiles, tiles, wg, wu, sg, su, expert_base, experts_local, I, H, 0, nullptr, act,
+                                 (cudaStream_t)stream);
     if (g_moe_mma && (rt == 1 || rt == 8) && !(H & 63) && !(I & 15) && !(xs & 7))
         return glmb_launch_moe_gateup_mma(x, xs, top_k, tile_expert, tile_routes, n_tiles, tiles, rt, wg, wu, sg, su, expert_base,
                                           experts_local, I, H, act, (cudaStream_t)stream);
@@ -267,6 +275,9 @@ GLMB_API int glmb_moe_down_fp8(const void* act, const float* route_weight, const
                                const int* n_tiles, int tiles, int rt, const void* wd, const float* sd, int expert_base,
                                int experts_local, int I, int H, void* dw, void* stream) {
     if ((I & 15) || tiles < 1) return 1;
+    if (g_moe_mma && rt == 8 && moe_tiles8_takes(act, I, wd, nullptr, dw, tile_routes, tiles, experts_local, H, I))
+        return launch_moe_tiles8(act, I, 1, tile_expert, tile_routes, n_tiles, tiles, wd, nullptr, sd, nullptr, expert_base, experts_local, H, I, 1,
+                                 route_weight, dw, (cudaStream_t)stream);
     if (g_moe_mma && (rt == 1 || rt == 8) && !(I & 63) && !(H & 15))
         return glmb_launch_moe_down_mma(act, route_weight, tile_expert, tile_routes, n_tiles, tiles, rt, wd, sd, expert_base, experts_local,
                                         I, H, dw, (cudaStream_t)stream);

@@ -593,10 +593,9 @@ class GlmMoeDsaModel:
             self.trace.setdefault("topk_ids", {})[layer] = ws.topk_ids[:rows].clone()
             self.trace.setdefault("topk_w", {})[layer] = ws.topk_w[:rows].clone()
         sort_kernel = self.route_sort_kernel and el <= 256 and ws.topk_ids[:rows].is_contiguous()
-        # The grouped GEMM reads an expert once however many routes it has and is the faster form at every count measured, gate/up + down of a
-        # layer of 256 experts: 200 rows 2,536 us (GEMV kernels on 8-route tiles) against 1,460, 300 rows 1,867 + 1,233 against 967 + 504, 380 rows
-        # 2,166 + 1,436 against 975 + 507; one rank's shard of eight, 300 rows: 231 + 187 against 130 + 98.  Chunks of up to 256 rows keep
-        # the GEMV kernels for one reason only: their launch program is recorded with them, and a changed one is accepted in a step of its own.
+        # Chunks of up to 256 rows keep tiles of eight routes, as their launch program is recorded; behind those entry points lies the same kernel as
+        # behind the grouped form, which gathers the rows itself (no copy in expert order: 200 rows 1,262 + 700 us a layer of 256 experts).  Longer
+        # chunks sort into tiles of 128 routes: 300 rows 967 + 504 us, on mma.sync tiles of eight 1,867 + 1,233.
         short = self.few_routes_rows is None or rows <= self.few_routes_rows
         few_per_expert = self.few_routes_gemv and sort_kernel and short and rows * tk < self.few_routes_limit * E
         if not decode and not few_per_expert and rows * tk >= 128 and H % 16 == 0 and I % 16 == 0:
