@@ -32,6 +32,5 @@ class LaneRegisters:
 
     def reset_lane(self, lane: int) -> None:
         """Fresh cache for a new request on ``lane`` (stale rows are never read: reads are bounded by the position)."""
-        self.positions[lane] = 0
-        self.tokens[lane] = 0
-        self.active[lane] = 0
+        for register in (self.positions, self.tokens, self.active):
+            register[lane].zero_()  # a launch; an assignment copies from the host, and waits for the copy
