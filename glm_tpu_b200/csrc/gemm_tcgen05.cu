@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "peer.cuh"
 #include "tcgen05.cuh"
+#include "gemm_few_tcgen05.cuh"
 #include "gemm_pair_tcgen05.cuh"
 
 #define TC_BM 128
@@ -502,6 +503,15 @@ static int gemm_pair_columns(int rows, int N, int* wave_cost = nullptr) {
     return best;
 }
 
+// Up to 256 rows: whether weights as M with K dealt to a cluster (gemm_few_tcgen05.cuh) are expected to be a microsecond faster than the form above
+// (8.4 us and its waves, of 24.6 us at K 4096).  More rows fill the other forms' tiles: [400 x 4096], K 12288: 51 us either way, [400 x 6144], K 4096:
+// 28.7 against 47.6.
+static bool gemm_few_takes(const GemmFewPlan& plan, int rows, int N, int K) {
+    int cost;
+    gemm_pair_columns(rows, N, &cost);
+    return plan.splits > 0 && plan.us + 1.0 < 8.4 + cost * (0.246 * K / 4096);
+}
+
 // a [rows, K] bf16 (lda), b [experts * N, K] bf16 (ldb), c [rows, N] bf16 or fp32 (ldc).  K % 8 == 0; a, b 16-byte
 // aligned with lda, ldb multiples of 8.  tiles / n_tiles: device arrays for grouped mode (max_tiles entries) or NULL.
 GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, int64_t ldb, void* c, int64_t ldc, int rows, int N,
@@ -516,6 +526,11 @@ GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, i
         int dev = 0;
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count < 1) sm_count = 148;
+    }
+    if (!tiles && rows <= 256 && (g_gemm_variant == 0 || (g_gemm_variant >= 16 && g_gemm_variant < 32))) {
+        const GemmFewPlan plan = gemm_few_plan(rows, N, K, g_gemm_variant ? g_gemm_variant - 16 : 0);
+        if (g_gemm_variant ? plan.splits > 0 : gemm_few_takes(plan, rows, N, K))
+            return launch_gemm_few(plan, a, lda, b, ldb, c, ldc, rows, N, K, out_f32, status, (cudaStream_t)stream);
     }
     const int bn = tiles ? 0 : g_gemm_variant >= 32 ? g_gemm_variant : g_gemm_variant == 0 ? gemm_pair_columns(rows, N) : 0;
     if (bn) return launch_gemm_pair(a, lda, b, nullptr, ldb, c, ldc, rows, N, K, bn, out_f32 ? GP_OUT_F32 : GP_OUT_BF16, 0, status, (cudaStream_t)stream);
@@ -546,7 +561,7 @@ GLMB_API int glmb_gemm_bf16_tcgen05(const void* a, int64_t lda, const void* b, i
 }
 
 // 0: choose by problem size; 1: always 128 x 128 tiles, one per CTA; 2: always the persistent 128 x 256 kernel; 128, 192, 256: dense problems on
-// pairs of SMs with so many columns per tile.
+// pairs of SMs with so many columns per tile; 16 + s: up to 256 rows, weights as M with K in s parts (16: as many as are expected to be best).
 GLMB_API void glmb_set_gemm_variant(int variant) { g_gemm_variant = variant; }
 
 // out[rows, N] (bf16, at comm->data[p] + out_offset on EVERY rank p) = sum over ranks of a_r[rows, K_r] . b_r[N, K_r]^T.
