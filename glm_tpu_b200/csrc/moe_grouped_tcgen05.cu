@@ -28,9 +28,9 @@
 //
 // Short prefill chunks bring their routes as tiles of eight (`moe_tiles8_*`, behind glmb_moe_gateup_fp8 / glmb_moe_down_fp8): neighbouring tiles of an
 // expert form an item of up to 64 routes, whose activations a warp of their own gathers.  All 256 experts, against a CTA per tile and 16 rows on mma.sync
-// (moe_gemv_mma.cu), which decodes an expert again for every eight routes: 60 rows (218 experts) 1,115 + 680 -> 976 + 523 us, 200 rows 1,497 + 933
-// -> 1,262 + 700, 256 rows 1,724 + 1,075 -> 1,294 + 703.  With the gather in warp 0, between the weights' copies, 1,544 + 810 (200 rows); with sixteen
-// decode warps on every step 1,346 + 705.
+// (moe_gemv_mma.cu), which decodes an expert again for every eight routes: 60 rows (218 experts) 1,115 + 680 -> 920 + 490 us, 200 rows 1,497 + 933
+// -> 1,131 + 620, 256 rows 1,724 + 1,075 -> 1,160 + 623.  On the way there, 60 rows: the gather in warp 0, between the weights' copies, 1,321 + 682; sixteen
+// decode warps on every step 1,128 + 582; a multiplication per code instead of one for two 976 + 523.
 // Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores (tiles of eight: stores NaN, their entry points
 // have no status word) and still frees its TMEM.
 //
@@ -333,8 +333,8 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                         const uint32_t c[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
 #pragma unroll
                         for (int p = 0; p < 4; ++p) {
-                            v[i * 8 + 2 * p] = dec2(c[p], scale);
-                            v[i * 8 + 2 * p + 1] = dec2(c[p] >> 16, scale);
+                            v[i * 8 + 2 * p] = dec2_packed(c[p], scale);
+                            v[i * 8 + 2 * p + 1] = dec2_packed(c[p] >> 16, scale);
                         }
                     }
                     __syncwarp();
