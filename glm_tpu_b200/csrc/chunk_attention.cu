@@ -599,6 +599,12 @@ static int launch_chunk_prefill(const ChunkAttnArgs& a, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
+// Several rows of eight key heads or more: 32 CTAs a row, whatever the number of rows (a row's sums do not depend on it), with rings of 100 KB (head sizes up
+// to 128), so that two CTAs share an SM and all are resident at once.  With rings of 200 KB and eight splits, 256 CTAs (four rows) ran in two
+// waves, and 128 in clusters of eight did not reach every SM: four chats at 1,000 (32 query heads over 8 key heads of 128) 27.0 -> 12.9 us, eight at
+// 3,000 34.4 -> 25.9, two at 3,000 23.8 -> 23.5.  With four key heads half as many CTAs fit one wave up to four rows: three chats at 700 9.7 us there, 10.4 here.
+static bool chunk_decode_many(const ChunkAttnArgs& a) { return a.rows > 1 && a.G * ceil_div(a.H / a.G, CD_HEADS) >= 8; }
+
 template <int DV, int WARPS, int NT>
 static int launch_chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
     static DeviceOnce once;
@@ -615,13 +621,15 @@ static int launch_chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
     const uint64_t ring_rows = (uint64_t)a.lanes * a.ring;
     if (make_map(&map_k, a.k, ring_rows, (uint64_t)a.G * a.dimp, (uint64_t)a.G * a.dimp, WARPS * 16)) return 3;
     if (make_map(&map_v, a.v, ring_rows, (uint64_t)a.G * a.vdimp, (uint64_t)a.G * a.vdimp, WARPS * 16)) return 3;
-    int stages = 4;
-    while (stages > 2 && chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS) > 200 * 1024) --stages;
-    // CTAs per cluster: enough that the grid reaches every SM, at least one tile each.  A cluster of 16 only while few are launched: the
-    // GPU places a handful of them at a time, and eight waited for one another (20 us before the first key, 10 us with eight per cluster).
     const int heads = a.G * ceil_div(a.H / a.G, CD_HEADS), tiles = ceil_div(a.ring, WARPS * 16), most = heads * a.rows <= 4 ? 16 : 8;
-    int splits = 1;
-    while (splits < most && splits * 2 <= tiles && splits * heads * a.rows < 148) splits *= 2;
+    const bool many = chunk_decode_many(a);
+    int stages = 4, splits = 1;
+    while (stages > 2 && chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS) > (many ? 104 : 200) * 1024) --stages;
+    if (many)
+        while (splits < 8 && splits * 2 <= tiles && splits * 2 * heads <= 32) splits *= 2;
+    else  // CTAs per cluster: enough that the grid reaches every SM, at least one tile each.  A cluster of 16 only while few are launched: the
+          // GPU places a handful of them at a time, and eight waited for one another (20 us before the first key, 10 us with eight per cluster).
+        while (splits < most && splits * 2 <= tiles && splits * heads * a.rows < 148) splits *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, heads, a.rows);
     cfg.blockDim = dim3(WARPS * 32);
@@ -663,6 +671,7 @@ GLMB_API int glmb_chunk_attn_decode(const ChunkAttnArgs* args, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (a.dimp > 128 || a.vdimp > 128) return few ? launch_chunk_decode<256, 4, 1>(a, st) : launch_chunk_decode<256, 4, 2>(a, st);
     if (a.vdimp <= 64) return few ? launch_chunk_decode<64, 8, 1>(a, st) : launch_chunk_decode<64, 8, 2>(a, st);
+    if (chunk_decode_many(a)) return few ? launch_chunk_decode<128, 4, 1>(a, st) : launch_chunk_decode<128, 4, 2>(a, st);
     return few ? launch_chunk_decode<128, 8, 1>(a, st) : launch_chunk_decode<128, 8, 2>(a, st);
 }
 
