@@ -135,7 +135,7 @@ static inline cudaError_t glmb_launch_carved(int carveout, void (*kernel)(KArgs.
 // large ring (attention, indexer: up to 200 KB) needed, and what is left of the L1, 28 KB, bounds the bytes in flight.  15 % is 32 KB of shared memory,
 // three CTAs.  Measured in captured decode steps on a B200: eight chats of the medium Namizen 1,573 -> 905 us a step ([4096 x 18432] 79 -> 30, head
 // [131072 x 4096] 340 -> 175), four of GLM at 5,000 1,875 -> 1,729, eight of the routed Zikevik 1,720 -> 1,557; with 8, 25 and 50 % 974, 971, 970 us for the
-// first.  Not for projections of one row (FMA): 25 % 1,058 -> 1,095 us in GLM, 15 % no change.
+// first.  Not for the FMA kernels of one row: 25 % 1,058 -> 1,095 us in GLM, 15 % no change.
 #define GLMB_L1_CARVEOUT 15
 #define GLMB_LAUNCH_L1(kernel, grid, block, smem, stream, ...) \
     (void)glmb_launch_carved(GLMB_L1_CARVEOUT, kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__)

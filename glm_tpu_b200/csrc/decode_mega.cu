@@ -319,9 +319,6 @@ __device__ __forceinline__ int mg_pick_ks(int units, int K, bool compat, int max
     return best;
 }
 
-// Whether a projection of `rows16` groups of 16 weight rows (a gate / up pair: 8 + 8) takes mg_gemv_mma, as the stand-alone kernels do.
-__host__ __device__ static inline bool mg_takes_mma(int rows, int rows16) { return rows > 1 && skinny_mma_takes(rows16); }
-
 // warp_dot_bf16 (gemv_core.cuh) with U steps of loads issued before their arithmetic: the same products added in the same
 // order, but 2 * U 16-byte loads in flight per lane, which the 16 resident warps of an SM need to keep HBM busy.
 template <int R, int U>
@@ -471,10 +468,10 @@ __device__ __forceinline__ void mg_gemv(int units, int K, int ks, int rows, MgSm
     }
 }
 
-// A projection of `rows16` groups of 16 weight rows with the sums of the stand-alone kernels.
+// A projection of `rows16` groups of 16 weight rows (a gate / up pair: 8 + 8) with the sums of the stand-alone kernels.
 template <int R, typename Get, typename Epi>
 __device__ __forceinline__ void mg_project(int rows16, int units, int K, int rows, MgSmall& sm, Get get, Epi epi) {
-    if (mg_takes_mma(rows, rows16)) mg_gemv_mma<R>(units, K, rows, sm, get, epi);
+    if (skinny_mma_takes(rows, rows16)) mg_gemv_mma<R>(units, K, rows, sm, get, epi);
     else mg_gemv<R>(units, K, mg_pick_ks(units, K, true, 0, 0), rows, sm, get, epi);
 }
 
@@ -660,7 +657,7 @@ template <int R>
 __device__ __forceinline__ void mg_gemv_allreduce(const bf16* x, int64_t xs, const bf16* w, int64_t ws, int N, int K, int rows, bf16* out,
                                                   int64_t os, int channel, const MegaArgs& a, MgSmall& sm) {
     const int units = (N + 1) / 2;
-    const bool mma = a.comm.world == 1 && mg_takes_mma(rows, (N + 15) / 16);  // the exchange of several GPUs stays with the FMA kernel (glmb_skinny_bf16)
+    const bool mma = a.comm.world == 1 && skinny_mma_takes(rows, (N + 15) / 16);  // the exchange of several GPUs stays with the FMA kernel (glmb_skinny_bf16)
     const int ks = mma ? 0 : mg_pick_ks(units, K, true, GLMB_AR_SLICE, 2 * R);
     const int tpc = mma ? MG_MMA_UNITS : MG_WARPS / ks;
     const int total_teams = gridDim.x * tpc;
@@ -1809,6 +1806,7 @@ __device__ __forceinline__ void mg_prefetch_own(const MegaArgs& a, const MegaLay
     }
 }
 
+#define MG_SM_SMEM (228 * 1024)
 // PHASE: 1..11 a layer's phases, 12 / 13 the head's two (a kernel per phase: its own registers, occupancy and code).
 // Resident CTAs per SM a phase kernel is compiled for: the streaming phases want many small CTAs (every byte of the table
 // requested at once), which bounds their registers; the tile phases keep the registers they need.
@@ -1816,7 +1814,7 @@ template <int R, bool COMPAT, int PHASE>
 struct MgPhaseBlocks {
     static constexpr bool streaming = PHASE == MG_QKV_A || PHASE == MG_Q_B || PHASE == MG_VPROJ || PHASE == MG_OPROJ || PHASE == MG_MLP_A ||
                                       PHASE == MG_MLP_B || PHASE == MG_COMBINE + MG_HEAD_LOGITS;
-    static constexpr int value = !streaming ? 2 : R > 4 ? 2 : (R > 2 || (COMPAT && R > 1)) ? 3 : 4;  // mg_gemv_mma: 80 registers
+    static constexpr int value = !streaming ? 2 : R > 4 ? 2 : (R > 2 || COMPAT) ? 3 : 4;  // mg_gemv_mma: 80 registers
 };
 
 template <int R, bool COMPAT, int PHASE>
@@ -1975,8 +1973,8 @@ static int host_pick_ks(int units, int K) {
     return ks;
 }
 // CTAs that give every unit of a projection its team of warps in one round (units: pairs of rows, or gate / up pairs)
-static int one_round(int rows, int rows16, int units, int K) {
-    const int per_cta = mg_takes_mma(rows, rows16) ? MG_MMA_UNITS : MG_WARPS / host_pick_ks(units, K);
+static int one_round(bool mma, int units, int K) {
+    const int per_cta = mma ? MG_MMA_UNITS : MG_WARPS / host_pick_ks(units, K);
     return (units + per_cta - 1) / per_cta;
 }
 
@@ -1987,20 +1985,21 @@ static int phase_grid(const MegaArgs& a, const MegaLayer& lw, int layer, int pha
     auto capped = [&](int ctas) { return ctas < 1 ? 1 : (ctas > GLMB_AR_MAX_CTAS ? GLMB_AR_MAX_CTAS : ctas); };
     const int H = a.H;
     // FMAs: many CTAs of few rows; fragments: one wave, every CTA normalises the step's rows first
-    if (layer >= a.num_layers) return phase != MG_HEAD_LOGITS ? 1 : a.compat_ksplit == 1 && !mg_takes_mma(a.rows, (a.vocab_local + 15) / 16) ? sms * 8 : wide;
+    if (layer >= a.num_layers) return phase != MG_HEAD_LOGITS ? 1 : a.compat_ksplit == 1 && !skinny_mma_takes(a.rows, (a.vocab_local + 15) / 16) ? sms * 8 : wide;
     if (a.compat_ksplit == 1) {
-        const int out_rows = a.comm.world == 1 ? a.rows : 1;  // projections with an exchange keep the FMA form (mg_gemv_allreduce)
+        auto mma = [&](int rows16) { return skinny_mma_takes(a.rows, rows16); };
+        const bool out_mma = a.comm.world == 1 && mma((H + 15) / 16);  // projections with an exchange keep the FMA form (mg_gemv_allreduce)
         switch (phase) {
-        case MG_QKV_A: return capped(one_round(a.rows, (lw.n_qkv_a + 15) / 16, (lw.n_qkv_a + 1) / 2, H));
-        case MG_Q_B: { const int g = one_round(a.rows, (lw.n_q_b + 15) / 16, (lw.n_q_b + 1) / 2, a.Q); return g < a.rows ? a.rows : g; }
-        case MG_OPROJ: return capped(one_round(out_rows, (H + 15) / 16, (H + 1) / 2, a.heads_local * a.vdim));
+        case MG_QKV_A: return capped(one_round(mma((lw.n_qkv_a + 15) / 16), (lw.n_qkv_a + 1) / 2, H));
+        case MG_Q_B: { const int g = one_round(mma((lw.n_q_b + 15) / 16), (lw.n_q_b + 1) / 2, a.Q); return g < a.rows ? a.rows : g; }
+        case MG_OPROJ: return capped(one_round(out_mma, (H + 1) / 2, a.heads_local * a.vdim));
         case MG_MLP_A: {
-            if (lw.dense) return capped(one_round(a.rows, (a.dense_cols + 7) / 8, a.dense_cols, H));
-            const int r = one_round(a.rows, (a.E + 15) / 16, (a.E + 1) / 2, H), sg = one_round(a.rows, (a.shared_cols + 7) / 8, a.shared_cols, H);
+            if (lw.dense) return capped(one_round(mma((a.dense_cols + 7) / 8), a.dense_cols, H));
+            const int r = one_round(mma((a.E + 15) / 16), (a.E + 1) / 2, H), sg = one_round(mma((a.shared_cols + 7) / 8), a.shared_cols, H);
             return capped(r > sg ? r : sg);
         }
         case MG_MLP_B:
-            if (lw.dense) return capped(one_round(out_rows, (H + 15) / 16, (H + 1) / 2, a.dense_cols));
+            if (lw.dense) return capped(one_round(out_mma, (H + 1) / 2, a.dense_cols));
             break;
         default: break;
         }
@@ -2047,11 +2046,19 @@ static int mega_phase_launch_one(const MegaArgs& a, const MegaLayer& lw, int lay
     cfg.blockDim = dim3(MG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = g_glmb_pdl_enabled ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    // The rest of the SM's memory is the L1 that the weights stream through (GLMB_LAUNCH_L1): a step of four GLM layers with one, two and four chats
+    // 1,810, 2,346 and 2,787 us without, 1,175, 1,640 and 2,228 with (one chat with FMAs, without: 1,373).
+    if (COMPAT && MgPhaseBlocks<R, COMPAT, PHASE>::streaming) {
+        const size_t share = ((smem + 1024) * occ[dev] * 100 + MG_SM_SMEM - 1) / MG_SM_SMEM;  // CTAs of one SM, each with the system's 1 KB
+        attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[1].val.sharedMemCarveout = share < 100 ? (unsigned)share : 100u;
+        cfg.numAttrs = 2;
+    }
     return (int)cudaLaunchKernelEx(&cfg, mega_phase_kernel<R, COMPAT, PHASE>, a, lw, layer, (int)big);
 }
 

@@ -152,7 +152,7 @@ skinny_bf16_kernel(const bf16* __restrict__ x, int64_t xs, int rows, const bf16*
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The same projection for two to eight rows (one problem, no exchange) with `skinny_mma_span` (gemv_core.cuh): 16 output features per CTA, K
+// The same projection (one problem, no exchange; `skinny_mma_takes`) with `skinny_mma_span` (gemv_core.cuh): 16 output features per CTA, K
 // split over its warps.
 template <int DEPTH>
 __global__ void __launch_bounds__(SK_THREADS, DEPTH == 4 ? 2 : 3)
@@ -294,7 +294,7 @@ GLMB_API int glmb_skinny_bf16(const void* x, int64_t xs, int rows, const void* w
     if (rows < 1 || rows > GLMB_MAX_ROWS || (K & 7) || (xs & 7) || (ws & 7) || (xb & 7) || (wb & 7) || batch < 1) return 1;
     PeerComm c = comm ? *comm : single_comm();
     const int groups = ceil_div(N, 16);
-    if (rows > 1 && skinny_mma_takes(groups) && batch == 1 && !(mode == SK_OUT_ALLREDUCE_BF16 && c.world > 1)) {
+    if (skinny_mma_takes(rows, groups) && batch == 1 && !(mode == SK_OUT_ALLREDUCE_BF16 && c.world > 1)) {
 #define CALL(D)                                                                                                                            \
     GLMB_LAUNCH_L1(skinny_mma_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)w, ws, N, K, out, os, mode, \
                 c.status, channel)
@@ -323,7 +323,7 @@ GLMB_API int glmb_skinny_bf16_swiglu(const void* x, int64_t xs, int rows, const 
                                      void* act, int64_t as, void* stream) {
     if (rows < 1 || rows > GLMB_MAX_ROWS || (K & 7) || (xs & 7) || (ws & 7)) return 1;
     const int groups = ceil_div(N, 8);
-    if (rows > 1 && skinny_mma_takes(groups)) {
+    if (skinny_mma_takes(rows, groups)) {
 #define CALL(D)                                                                                                                                   \
     GLMB_LAUNCH_L1(skinny_mma_swiglu_kernel<D>, groups, SK_THREADS, 0, (cudaStream_t)stream, (const bf16*)x, xs, rows, (const bf16*)wg, (const bf16*)wu, ws, \
                 N, K, (bf16*)act, as)

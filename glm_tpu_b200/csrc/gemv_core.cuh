@@ -80,9 +80,9 @@ __device__ __forceinline__ void warp_reduce_all(float (&acc)[NPW][R]) {
 
 // ---------------------------------------------------------------------------------------------------
 // 16 weight rows as the M and one to eight activation rows as the N of mma.sync m16n8k16 (bf16 products, fp32 sums).  A row's bits depend neither on
-// how many others there are (from two rows on) nor on what they hold; a row alone takes the FMA kernel, which adds in another order.  With R rows the
+// how many others there are nor on what they hold, where a row alone takes these kernels too.  With R rows the
 // FMA loop above issues R + 2 instructions per weight and is bound by issue from four rows on; here a weight costs a sixteenth of an
-// instruction whatever R is, and nothing is shuffled at the end.  Measured on a B200, [6144 x 16384]: 2 rows 49.8 -> 32.2 us, 4 rows
+// instruction whatever R is, and nothing is shuffled at the end.  Measured on a B200 (launches of their own), [6144 x 16384]: 2 rows 49.8 -> 32.2 us, 4 rows
 // 58.0 -> 32.6, 8 rows 85.5 -> 32.9 (6.1 TB/s); [131072 x 4096]: 193 -> 154, 218 -> 158, 397 -> 163.
 //
 // The tensor core truncates what it adds to an accumulator, so every instruction starts from zero and its sixteen products' sum is added in
@@ -141,9 +141,11 @@ __device__ __forceinline__ void skinny_mma_span(const bf16* w_lo, const bf16* w_
     skinny_mma_chunks<DEPTH>(w_lo, w_hi, xr, K, warp, SKM_WARPS, (K + 63) >> 6, t, c);
 }
 
-// Whether a projection of so many groups of 16 weight rows takes the kernels above: a CTA has one group, and fewer than 64 CTAs leave the
-// machine idle ([256 x 6144]: 16 CTAs 4.8 us, the FMA kernel's 128 CTAs of two rows 3.1; [2048 x 2048]: 3.8 against 4.4).
-__host__ __device__ static inline bool skinny_mma_takes(int groups) { return groups >= 64; }
+// Whether a projection of so many groups of 16 weight rows takes the kernels above: a CTA has one group.  Fewer than 64 CTAs leave the
+// machine idle ([256 x 6144]: 16 CTAs 4.8 us, the FMA kernel's 128 CTAs of two rows 3.1; [2048 x 2048]: 3.8 against 4.4).  A row alone, in a step: from a CTA
+// per SM on ([6144 x 16384] 36.0 -> 31.5 us, [2624 x 6144] 7.9 -> 6.8, [154880 x 6144] 273 -> 261, [4096 x 14336] 25.6 -> 19.8); with 128 the FMA
+// kernel's smaller CTAs are done as early and let the next kernel in earlier ([2048 x 10240] 10.5 against 11.1).
+__host__ __device__ static inline bool skinny_mma_takes(int rows, int groups) { return groups >= (rows > 1 ? 64 : 148); }
 
 // Chunks in flight per warp: four with two CTAs per SM, or two with three.  The last wave decides: whichever fills its waves better ([4096 x
 // 18432], 256 CTAs: 25.4 against 28.0 us; [6144 x 16384], 384 CTAs: 37.4 against 32.6).  Rows of fewer than two rounds of

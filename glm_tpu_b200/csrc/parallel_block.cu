@@ -120,53 +120,6 @@ __device__ __forceinline__ void dp_prefetch(const void* rows, int64_t bytes) {
     if (threadIdx.x == 0 && n) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rows), "r"(n) : "memory");
 }
 
-// One row.  Blocks [0, proj_blocks): out[n] = x1 . w[n] (two output columns per warp group); the others: act[n] = f(x2 . wg[n]) * (x2 . wu[n]).
-// ks warps of a CTA split K for the same outputs.  Weight rows are contiguous ([N, K]).
-__global__ void __launch_bounds__(DP_THREADS)
-dual_proj_row_kernel(const bf16* __restrict__ x1, const bf16* __restrict__ x2, int K, const bf16* __restrict__ w, int N, bf16* __restrict__ out,
-                     const bf16* __restrict__ wg, const bf16* __restrict__ wu, int F, bf16* __restrict__ act, int kind, int proj_blocks, int ks) {
-    asm volatile("griddepcontrol.launch_dependents;");
-    const bool gated = (int)blockIdx.x >= proj_blocks;
-    const int groups = DP_WARPS / ks;
-    if (!gated) {
-        const int first = blockIdx.x * groups * 2;
-        dp_prefetch(w + (int64_t)first * K, (int64_t)min(groups * 2, N - first) * K * 2);
-    } else {
-        const int first = (blockIdx.x - proj_blocks) * groups, count = min(groups, F - first);
-        dp_prefetch(wg + (int64_t)first * K, (int64_t)count * K * 2);
-        dp_prefetch(wu + (int64_t)first * K, (int64_t)count * K * 2);
-    }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    __shared__ float red[DP_WARPS][2];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int group = warp / ks, kpart = warp % ks;
-    const int n = gated ? (blockIdx.x - proj_blocks) * groups + group : (blockIdx.x * groups + group) * 2;
-    const bool valid = n < (gated ? F : N);
-    const bf16* const xr[1] = {gated ? x2 : x1};
-    float acc[2][1] = {{0.f}, {0.f}};
-    if (valid) {
-        const bf16* wp[2] = {gated ? wg + (int64_t)n * K : w + (int64_t)n * K, gated ? wu + (int64_t)n * K : w + (int64_t)min(n + 1, N - 1) * K};
-        const int kspan = K / ks;
-        warp_dot_bf16<1, 2>(xr, wp, kpart * kspan, (kpart + 1) * kspan, lane, acc);
-        warp_reduce_all<1, 2>(acc);
-    }
-    if (ks > 1) {
-        if (lane == 0) { red[warp][0] = acc[0][0]; red[warp][1] = acc[1][0]; }
-        __syncthreads();
-        if (kpart == 0 && lane == 0)
-            for (int p = 1; p < ks; ++p) { acc[0][0] += red[warp + p][0]; acc[1][0] += red[warp + p][1]; }
-    }
-    if (lane == 0 && kpart == 0 && valid) {
-        if (gated) {
-            act[n] = __float2bfloat16_rn(glu_activation(kind, acc[0][0]) * acc[1][0]);
-        } else {
-            out[n] = __float2bfloat16_rn(acc[0][0]);
-            if (n + 1 < N) out[n + 1] = __float2bfloat16_rn(acc[1][0]);
-        }
-    }
-}
-
-// Two to eight rows.
 // Blocks [0, proj_blocks): out[r][n] = x1[r] . w[n]                        (16 output columns)
 // the others:              act[r][n] = f(x2[r] . wg[n]) * (x2[r] . wu[n])  (8 output columns: 8 gate rows over their 8 up rows)
 // The warps of a CTA split K (`skinny_mma_span`, gemv_core.cuh).  Weight rows are contiguous ([N, K]).
@@ -231,19 +184,11 @@ GLMB_API int glmb_parallel_norm(const int* tokens, const void* table, int vocab,
     return (int)cudaGetLastError();
 }
 
-// bf16, 1..8 rows.  F = 0: projection only.  K a multiple of 8, w [N, K] and wg / wu [F, K] contiguous.
+// bf16, 1..8 rows (one row with FMAs and warps per output instead, [6144 + 2 x 14336 x 4096] in a step: 43.6 us against 45.0, and the projection behind it 38.6
+// against 28.4).  F = 0: projection only.  K a multiple of 8, w [N, K] and wg / wu [F, K] contiguous.
 GLMB_API int glmb_dual_proj(const void* x1, const void* x2, int64_t xs, int rows, int K, const void* w, int N, void* out, int64_t os,
                             const void* wg, const void* wu, int F, void* act, int64_t as, int kind, void* stream) {
     if (rows < 1 || rows > GLMB_MAX_ROWS || (K & 7) || K < 8 || (xs & 7) || N < 1 || F < 0 || (kind != GLU_SILU && kind != GLU_GELU_TANH)) return 1;
-    if (rows == 1) {  // [3072 + 2 x 8192] x 2048 in a decode step of six layers: 311 us a step, 317 with the kernel below
-        const int units = ceil_div(N, 2) + F;
-        int ks = 1;  // enough warps per output that about four CTAs land on every SM, with at least 256 columns per warp
-        while (ks < DP_WARPS && units * ks < 148 * 4 * DP_WARPS && K % (ks * 2 * 8) == 0 && K / (ks * 2) >= 256) ks *= 2;
-        const int teams = DP_WARPS / ks, proj_blocks = ceil_div(N, teams * 2);
-        GLMB_LAUNCH(dual_proj_row_kernel, proj_blocks + ceil_div(F, teams), DP_THREADS, 0, (cudaStream_t)stream, (const bf16*)x1, (const bf16*)x2, K,
-                    (const bf16*)w, N, (bf16*)out, (const bf16*)wg, (const bf16*)wu, F, (bf16*)act, kind, proj_blocks, ks);
-        return (int)cudaGetLastError();
-    }
     const int proj_blocks = ceil_div(N, 16), grid = proj_blocks + ceil_div(F, 8);
 #define CALL(D)                                                                                                                                      \
     GLMB_LAUNCH_L1(dual_proj_kernel<D>, grid, DP_THREADS, 0, (cudaStream_t)stream, (const bf16*)x1, (const bf16*)x2, xs, rows, K, (const bf16*)w, N, (bf16*)out, \
