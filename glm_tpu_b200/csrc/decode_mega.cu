@@ -2051,8 +2051,8 @@ static int mega_phase_launch_one(const MegaArgs& a, const MegaLayer& lw, int lay
     attr[0].val.programmaticStreamSerializationAllowed = g_glmb_pdl_enabled ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // The rest of the SM's memory is the L1 that the weights stream through (GLMB_LAUNCH_L1): a step of four GLM layers with one, two and four chats
-    // 1,810, 2,346 and 2,787 us without, 1,175, 1,640 and 2,228 with (one chat with FMAs, without: 1,373).
+    // The rest of the SM's memory is the L1 that the weights stream through (GLMB_LAUNCH_L1): a step of four GLM layers with two and four chats 2,355
+    // and 2,888 us without, 1,640 and 2,228 with; eight layers and one chat 3,662 without, where FMAs took 2,772 (four layers: 1,175 with, FMAs 1,373).
     if (COMPAT && MgPhaseBlocks<R, COMPAT, PHASE>::streaming) {
         const size_t share = ((smem + 1024) * occ[dev] * 100 + MG_SM_SMEM - 1) / MG_SM_SMEM;  // CTAs of one SM, each with the system's 1 KB
         attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;

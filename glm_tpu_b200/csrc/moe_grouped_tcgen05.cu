@@ -14,17 +14,17 @@
 //                weight-decode contract), into TENSOR MEMORY, which the tensor core reads as its A operand: decoded weights that went
 //                through shared memory (64 KB written and 64 KB read a step) were what bound this kernel.  Two stages per matrix
 //   warp 1       issues tcgen05.mma (two matrices of M 128, N 16 .. 128)
-//   warps 2-5    epilogue of the tile before, while the next one is decoded and multiplied: a thread owns a weight row (TMEM lane)
+//   warps 2-5    epilogue (more than 64 routes: a fifth of it) of the tile before, while the next one is decoded and multiplied: a thread owns a weight row (TMEM lane)
 //                  gate/up mode  act = bf16( silu(bf16 gate) * bf16 up ), stored in sorted order
 //                  down mode     dw[route] = bf16( bf16(acc) * bf16(route weight) ), scattered to the route's slot
 //
 // TMEM: 256 columns of accumulators (two tiles of up to 64 routes, or one of more), 256 of decoded weights.
 //
-// What bounds it: the FP8 bytes, which cross HBM once (5.0 - 5.6 TB/s up to 777 rows), and with many routes the epilogue of tiles of more than
-// 64 routes, which have one accumulator.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 1,061 + 554 us
-// (a kernel with the routes as the M and decoded weights in shared memory: 1,931 + 1,065); 2,048 rows 1,413 + 799 us (2,377 + 1,302) with an
-// approximate quotient in the activation.  The exact one, whose results are those of the other forms of this projection bit for bit, costs 6 % (1,247
-// against 1,174 us a launch, both directions, in a prompt of 4,096 tokens).
+// What bounds it: the FP8 bytes, which cross HBM once (5.3 - 5.8 TB/s up to 777 rows), and with many routes the decode, which is done again for every 128
+// routes of an expert, and the activations from L2.  A tile of more than 64 routes has all the accumulators, so the next one waits for its epilogue: the decode
+// warps, idle then, store four fifths of it.  Measured on a B200, [256 experts, 2 x 2048 x 6144] and back, 219 experts chosen: 777 rows 980 + 516 us
+// (a kernel with the routes as the M and decoded weights in shared memory: 1,931 + 1,065), 2,048 rows 1,302 + 702 us (2,377 + 1,302); with the epilogue to
+// four warps alone 2,048 rows 1,417 + 772, 128 routes for every expert 1,818 + 1,001 against 1,626 + 905.
 //
 // Short prefill chunks bring their routes as tiles of eight (`moe_tiles8_*`, behind glmb_moe_gateup_fp8 / glmb_moe_down_fp8): neighbouring tiles of an
 // expert form an item of up to 64 routes, whose activations a warp of their own gathers.  All 256 experts, against a CTA per tile and 16 rows on mma.sync
@@ -51,6 +51,7 @@
 #define MG_TILE8_THREADS (MG_THREADS + 32)
 #define MG_RAW 4       // FP8 weights: 128 rows x 128 bytes of each matrix
 #define MG_CONV_WARPS 16
+#define MG_TEAMS (1 + MG_CONV_WARPS / 4)  // sets of four warps that store a tile of more than 64 routes
 #define MG_THREADS (6 * 32 + 32 * MG_CONV_WARPS)
 #define MG_SMEM_BYTES ((MG_STAGES * 2 + MG_RAW * 2) * MG_BOX + 1024)
 #define MG_TILE8_SMEM_BYTES (MG_TILE8_STAGES * 2 * MG_TILE8_BOX + MG_RAW * 2 * MG_BOX + MG_LIST * 4 + 1024)
@@ -133,6 +134,49 @@ __device__ __forceinline__ int mg_list_pieces(const MoeGroupedArgs& a, int n, ui
     return pieces;
 }
 
+// Results of 16 routes from `r0` on for this warp's 32 weight rows: thread = weight row = TMEM lane; neighbouring lanes swap, so that each stores two columns
+// of one route.  route16 / weight16: of column r0 + lane % 16 (-1: none).
+template <bool TILES8>
+__device__ __forceinline__ void mg_store16(const MoeGroupedArgs& a, uint32_t d0, uint32_t d1, int r0, int routes, int row0, int n0, int lane, int route16,
+                                           float weight16) {
+    if (a.mode == 0) {
+        uint32_t g[16], u[16];
+        tmem_ld16(d0 + r0, g);
+        tmem_ld16(d1 + r0, u);
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+            float v[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float gv = bf16_round(__uint_as_float(g[e + q])), uv = bf16_round(__uint_as_float(u[e + q]));
+                v[q] = gv * sigmoidf_precise(gv) * uv;
+            }
+            const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[0] : v[1], 1);
+            const int r = r0 + e + (lane & 1);
+            const int to = TILES8 ? __shfl_sync(0xffffffffu, route16, e + (lane & 1)) : r < routes ? row0 + r : -1;
+            if (to >= 0 && n0 < a.N)
+                *reinterpret_cast<uint32_t*>(a.out + (int64_t)to * a.N + n0) = (lane & 1) ? pack_bf16(got, v[1]) : pack_bf16(v[0], got);
+        }
+    } else {
+        uint32_t x[2][16];
+        tmem_ld16(d0 + r0, x[0]);
+        tmem_ld16(d1 + r0, x[1]);
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+            const int to = __shfl_sync(0xffffffffu, route16, e + (lane & 1));
+            const float w0 = __shfl_sync(0xffffffffu, weight16, e), w1 = __shfl_sync(0xffffffffu, weight16, e + 1);
+            bf16* dst = a.out + (int64_t)to * a.N + n0;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float v0 = bf16_round(__uint_as_float(x[m][e])) * w0, v1 = bf16_round(__uint_as_float(x[m][e + 1])) * w1;
+                const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v0 : v1, 1);
+                if (to >= 0 && n0 + m * 128 < a.N)
+                    *reinterpret_cast<uint32_t*>(dst + m * 128) = (lane & 1) ? pack_bf16(got, v1) : pack_bf16(v0, got);
+            }
+        }
+    }
+}
+
 // TILES8: the routes come as tiles of eight (row lists) instead of sorted rows, and their activations are gathered by warp 22 with cp.async.
 template <bool TILES8>
 __global__ void __launch_bounds__(TILES8 ? MG_TILE8_THREADS : MG_THREADS, 1)
@@ -141,7 +185,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     GLMB_PDL_PROLOGUE();
     constexpr int STAGES = TILES8 ? MG_TILE8_STAGES : MG_STAGES, XBOX = TILES8 ? MG_TILE8_BOX : MG_BOX;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t x_full[STAGES], x_empty[STAGES], raw_full[MG_RAW], raw_empty[MG_RAW], w_full[4], w_empty[4], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t x_full[STAGES], x_empty[STAGES], raw_full[MG_RAW], raw_empty[MG_RAW], w_full[4], w_empty[4], acc_full[2], acc_empty[2], wide_full, wide_done;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t fail;
     __shared__ int warp_counts[MG_TILE8_THREADS / 32];
@@ -168,6 +212,8 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         for (int s = 0; s < MG_RAW; ++s) { mbar_init(raw_full + s, 1); mbar_init(raw_empty + s, MG_CONV_WARPS / 2); }
         for (int j = 0; j < 4; ++j) { mbar_init(w_full + j, MG_CONV_WARPS / 4); mbar_init(w_empty + j, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4); }
+        mbar_init(&wide_full, 1);
+        mbar_init(&wide_done, MG_CONV_WARPS);
         fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -254,7 +300,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         __syncwarp();
         if (ok && g > 0 && lane == 0) mbar_arrive(x_full + (g - 1) % STAGES);
     } else if (warp == 1) {
-        uint32_t g = 0;
+        uint32_t g = 0, wides = 0;
         MgHalves at;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const TcTile t = tile_of(it);
@@ -265,6 +311,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
             for (int h = 0; h < 2; ++h)
                 if (ok && at.takes(h) && at.uses[h] > 0) ok = mbar_wait_warp(acc_empty + h, (at.uses[h] - 1) & 1);
+            if (ok && wides > 0) ok = mbar_wait_warp(&wide_done, (wides - 1) & 1);
             if (!ok) { fail = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int kb = 0; kb < steps && ok; ++kb, ++g) {
@@ -292,9 +339,11 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             if (elect_one()) {  // complete, or abandoned after a timeout: either way release the epilogue
                 if (at.takes(0)) umma_commit(acc_full);
                 if (at.takes(1)) umma_commit(acc_full + 1);
+                if (at.wide) umma_commit(&wide_full);
             }
             __syncwarp();
             if (!ok) break;
+            wides += at.wide;
             at.done();
         }
     } else if (warp >= 6) {
@@ -310,7 +359,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             const int n0 = (it % blocks) * cols + (a.mode == 1 ? m * 128 : 0);
             return scales + ((int64_t)tile_of(it).expert * n_srows + min(n0 >> 7, n_srows - 1)) * n_scols;
         };
-        uint32_t g = 0;
+        uint32_t g = 0, wides = 0;
         bool ok = true, asked = false;
         float next = 0.f;  // the scale of this set's next step, asked for a step ahead
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
@@ -351,9 +400,32 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(w_full + m * 2 + j);
             }
+            if constexpr (!TILES8) {
+                // A tile of more than 64 routes has all the accumulators, so the next one waits for its epilogue: these warps, which have nothing to decode
+                // for meanwhile, take four of every five pieces of 16 routes
+                const TcTile t = tile_of(it);
+                const int routes = min(t.row_end - t.row0, MG_ROUTES), n0 = (it % blocks) * cols + quarter * 32 + (lane & ~1);
+                if (routes <= 64 || !ok) continue;
+                const bool done = mbar_wait_warp(&wide_full, wides++ & 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!done || __any_sync(0xffffffffu, fail)) {
+                    fail = 1;
+                    if (lane == 0) raise_status(a.status, GLMB_STATUS_WAIT_TIMEOUT);
+                    break;
+                }
+                const uint32_t d = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+                for (int r0 = (set + 1) * 16; r0 < routes; r0 += MG_TEAMS * 16) {
+                    const int r = r0 + (lane & 15), route = r < routes && a.mode == 1 ? a.perm[t.row0 + r] : -1;
+                    mg_store16<TILES8>(a, d, d + 128, r0, routes, t.row0, n0, lane, route, route >= 0 ? bf16_round(a.route_weight[route]) : 0.f);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&wide_done);
+            }
         }
     } else {
-        // ---- epilogue: thread = weight row = TMEM lane; neighbouring lanes swap, so that each stores two columns of one route -----------
+        // ---- epilogue -----------
         const int quarter = warp & 3;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         MgHalves at;
@@ -388,46 +460,11 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             }
             const uint32_t d0 = tmem + lanes + at.column(0), d1 = tmem + lanes + at.column(1);
 #pragma unroll 1
-            for (int r0 = 0; r0 < routes; r0 += 16) {
-                if (a.mode == 0) {
-                    uint32_t g[16], u[16];
-                    tmem_ld16(d0 + r0, g);
-                    tmem_ld16(d1 + r0, u);
-#pragma unroll
-                    for (int e = 0; e < 16; e += 2) {
-                        float v[2];
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            const float gv = bf16_round(__uint_as_float(g[e + q])), uv = bf16_round(__uint_as_float(u[e + q]));
-                            v[q] = gv * sigmoidf_precise(gv) * uv;
-                        }
-                        const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[0] : v[1], 1);
-                        const int r = r0 + e + (lane & 1);
-                        const int to = TILES8 ? __shfl_sync(0xffffffffu, r0 < 32 ? route[0] : route[1], r & 31) : r < routes ? t.row0 + r : -1;
-                        if (to >= 0 && n0 < a.N)
-                            *reinterpret_cast<uint32_t*>(a.out + (int64_t)to * a.N + n0) = (lane & 1) ? pack_bf16(got, v[1]) : pack_bf16(v[0], got);
-                    }
-                } else {
-                    const int q = r0 >> 5, at32 = r0 & 31;
-                    const int routes32 = q < 2 ? (q ? route[1] : route[0]) : (q & 1 ? route[3] : route[2]);
-                    const float weights32 = q < 2 ? (q ? weight[1] : weight[0]) : (q & 1 ? weight[3] : weight[2]);
-                    uint32_t x[2][16];
-                    tmem_ld16(d0 + r0, x[0]);
-                    tmem_ld16(d1 + r0, x[1]);
-#pragma unroll
-                    for (int e = 0; e < 16; e += 2) {
-                        const int to = __shfl_sync(0xffffffffu, routes32, at32 + e + (lane & 1));
-                        const float w0 = __shfl_sync(0xffffffffu, weights32, at32 + e), w1 = __shfl_sync(0xffffffffu, weights32, at32 + e + 1);
-                        bf16* dst = a.out + (int64_t)to * a.N + n0;
-#pragma unroll
-                        for (int m = 0; m < 2; ++m) {
-                            const float v0 = bf16_round(__uint_as_float(x[m][e])) * w0, v1 = bf16_round(__uint_as_float(x[m][e + 1])) * w1;
-                            const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v0 : v1, 1);
-                            if (to >= 0 && n0 + m * 128 < a.N)
-                                *reinterpret_cast<uint32_t*>(dst + m * 128) = (lane & 1) ? pack_bf16(got, v1) : pack_bf16(v0, got);
-                        }
-                    }
-                }
+            for (int r0 = 0; r0 < routes; r0 += at.wide ? MG_TEAMS * 16 : 16) {  // a tile of more than 64 routes: the decode warps take the others
+                const int q = r0 >> 5, from = (r0 & 31) + (lane & 15);
+                const int route16 = __shfl_sync(0xffffffffu, q < 2 ? (q ? route[1] : route[0]) : (q & 1 ? route[3] : route[2]), from);
+                const float weight16 = __shfl_sync(0xffffffffu, q < 2 ? (q ? weight[1] : weight[0]) : (q & 1 ? weight[3] : weight[2]), from);
+                mg_store16<TILES8>(a, d0, d1, r0, routes, t.row0, n0, lane, route16, weight16);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
