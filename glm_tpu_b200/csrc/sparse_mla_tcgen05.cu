@@ -10,13 +10,17 @@
 // heads, and a thread of the softmax owns a key (a TMEM lane) with the scores of half the heads.
 //
 //   warps 0-7   softmax: scores from TMEM (two threads per key, 32 heads each), weights to shared memory, output of a finished row
-//   warps 8-11  gather: cp.async of the selected rows into nine 128-key x 64-column boxes (128-byte swizzle); queries by TMA
+//   warps 8-11  gather: cp.async of the selected rows into nine 128-key x 64-column boxes (128-byte swizzle); queries by TMA.  Then, while the
+//               weights are made, the output so far is scaled to the new maxima
 //   warp 12     issues every tcgen05.mma, owns the TMEM
 //
 // What bounds it: the gather (147 KB per 128 keys and row out of L2) and the chain gather -> S -> softmax -> O of a block, because the
-// queries (72 KB) leave room for one block of keys.  The chain is shortened by freeing the boxes two by two: the next block's
-// first columns are on their way while the last columns of this block are still being multiplied.  The weights lie where
-// the rotary columns were, which the second product does not need.
+// queries (72 KB) leave room for one block of keys.  The chain is shortened by freeing the boxes two by two and handing them on two by two: the next
+// block's first columns are on their way, and multiplied with the queries, while the last columns of this block are still in use.  The weights lie where
+// the rotary columns were, which the second product does not need.  Of 10.6 k clocks a block (128 keys) the gather waited 7.2 k for boxes to be freed
+// and the softmax worked 3.0 k, a quarter of that on the output's scale, which changes in nine blocks of ten; a row's division and stores took 14.5 k.
+// 2,048 rows of 2,048 keys: 1,276 us; pairs handed on as they arrive, not behind the last copy that is asked for, 1,126 (two pairs later 1,173; eight
+// gather warps, which leave the softmax 96 registers, 1,181); with the scaling in the gather warps and divisions without branches 1,009.
 //
 // Weights are taken relative to the running maximum of their head, block by block, as in sparse_mla_rows_kernel (which takes every other
 // shape): the heaviest weight is then 1 and loses nothing when the weights enter the second product as bf16.  A reference that lags behind by up
@@ -25,7 +29,7 @@
 // sums are fp32.
 //
 // Rows are dealt to one CTA per SM, longest (last) first.  2,048 rows of 2,048 keys on a B200: 5.27 ms with sparse_mla_rows_kernel (111 TFLOP/s),
-// 1.28 ms here (460 TFLOP/s; 1.04 with a lagging reference and a reciprocal); 777 rows 0.55 ms; 24 rows: 170 -> 97 us; 200 rows of 200 keys: 84 -> 36.
+// 1.01 ms here (579 TFLOP/s); 777 rows 0.44 ms; 64 rows 79 us; 200 rows of 200 keys: 84 -> 26.
 //
 // Every wait is bounded; a wait that runs out raises GLMB_STATUS_WAIT_TIMEOUT and the CTA still releases its TMEM.
 #include "attention_core.cuh"
@@ -67,6 +71,12 @@ __device__ __forceinline__ float sm_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// a / b, correctly rounded (the contract divides), of y = the rounded 1 / b: a quotient and one correction by its remainder (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000", theorem 8.5), without the branch of a division.  Infinities keep the first quotient.
+__device__ __forceinline__ float sm_quotient(float a, float b, float y) {
+    const float q = a * y, exact = fmaf(fmaf(-q, b, a), y, q);
+    return exact == exact ? exact : q;
+}
 __device__ __forceinline__ void sm_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 struct SparseMlaArgs {
     const bf16* kv_cache;
@@ -82,8 +92,8 @@ struct SparseMlaArgs {
 __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __grid_constant__ CUtensorMap map_q, SparseMlaArgs a) {
     GLMB_PDL_PROLOGUE();  // before the TMEM allocation: a kernel still running may need the columns to finish
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(16) float top_s[8][SM_HALF], ref_s[8][SM_HALF], fix_s[8][SM_HALF], sum_s[8][SM_HALF];  // per softmax warp and head of its half
-    __shared__ __align__(8) uint64_t q_full, k_full[5], s_full, p_full, o_done[4];
+    __shared__ __align__(16) float top_s[8][SM_HALF], ref_s[8][SM_HALF], fix_s[8][SM_HALF], sum_s[8][SM_HALF], inv_s[8][SM_HALF];  // per softmax warp and head of its half
+    __shared__ __align__(8) uint64_t q_full, k_full[5], s_full, fix_full, p_full, o_done[4];
     __shared__ uint32_t tmem_slot;
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     unsigned char* k_s = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -91,7 +101,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
     unsigned char* p_s = k_s + (SM_BOXES - 1) * SM_KBOX;  // the rotary box
 
     if (threadIdx.x == 0) {
-        mbar_init(&q_full, 1); mbar_init(&s_full, 1); mbar_init(&p_full, 8);
+        mbar_init(&q_full, 1); mbar_init(&s_full, 1); mbar_init(&fix_full, 2); mbar_init(&p_full, 12);
         for (int i = 0; i < 5; ++i) mbar_init(k_full + i, 4);
         for (int i = 0; i < 4; ++i) mbar_init(o_done + i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -123,6 +133,11 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
             next_start += SM_KEYS;
         };
         fetch();
+        auto hand_on = [&](int j) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies -> visible to the tensor core
+            __syncwarp();
+            if (lane == 0) mbar_arrive(k_full + j);
+        };
         bool ok = true;
         for (int i = blockIdx.x; i < a.rows && ok; i += gridDim.x) {
             const int r = a.rows - 1 - i, count = keys_of(r);
@@ -152,19 +167,37 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
                                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src[e] + b * 64), "r"(key0 + 16 * e < cnt ? 16 : 0) : "memory");
                             }
                     asm volatile("cp.async.commit_group;" ::: "memory");
+                    if (j > 0) {  // a pair is handed on when the next one has been asked for: the products with it run while later boxes are still in use
+                        asm volatile("cp.async.wait_group 1;" ::: "memory");
+                        hand_on(j - 1);
+                    }
                 }
                 if (!ok) break;
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                hand_on(4);
+                // ---- the output so far to the new maxima of its heads, while the softmax warps make the weights: nothing is to be copied meanwhile
+                if (start > 0) {
+                    if (!mbar_wait_warp(&fix_full, n & 1)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                    for (int half = 0; half < 2; ++half) {
+                        const float* fix = fix_s[half * 4];
+                        if (!__any_sync(0xffffffffu, fix[lane] != 1.f)) continue;
+                        const uint32_t o_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 + half * SM_HALF;
+#pragma unroll 1
+                        for (int c = 0; c < SM_L / 2; c += 64) {
+                            float o[SM_HALF];
+                            sm_ld32(o_addr + c, o);
 #pragma unroll
-                for (int j = 0; j < 5; ++j) {
-                    if (j == 0) asm volatile("cp.async.wait_group 4;" ::: "memory");
-                    if (j == 1) asm volatile("cp.async.wait_group 3;" ::: "memory");
-                    if (j == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-                    if (j == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                    if (j == 4) asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies -> visible to the tensor core
+                            for (int e = 0; e < SM_HALF; ++e) o[e] *= fix[e];
+                            sm_st32(o_addr + c, o);
+                        }
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(k_full + j);
                 }
+                if (lane == 0) mbar_arrive(&p_full);
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -251,19 +284,10 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
                 ref[lane] = next == -INFINITY ? 0.f : next;
                 run = next;
                 __syncwarp();
-                if (__any_sync(0xffffffffu, factor != 1.f) && start > 0) {  // the products of the block before are complete: the scores of this one follow them
+                if (lane == 0 && (warp & 3) == 0) mbar_arrive(&fix_full);  // the products of the block before are complete: the scores of this one follow them
+                if (__any_sync(0xffffffffu, factor != 1.f) && start > 0)
 #pragma unroll
                     for (int h = 0; h < SM_HALF; ++h) l[h] *= fix[h];
-#pragma unroll 1
-                    for (int c = 0; c < SM_L / 2; c += 64) {
-                        float o[32];
-                        sm_ld32(o_addr + c, o);
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) o[e] *= fix[e];
-                        sm_st32(o_addr + c, o);
-                    }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                }
 #pragma unroll
                 for (int c = 0; c < SM_HALF; c += 8) {
                     const float4 m0 = *reinterpret_cast<const float4*>(ref + c), m1 = *reinterpret_cast<const float4*>(ref + c + 4);
@@ -297,7 +321,11 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
             sum_s[warp][lane] = l[0];
             sm_barrier();
             const float (*sums)[SM_HALF] = sum_s + half * 4;
-            fix[lane] = (sums[0][lane] + sums[1][lane]) + (sums[2][lane] + sums[3][lane]);
+            // (in arrays of this warp that nobody else reads: `fix` may still be in use, and the sums are)
+            const float total = (sums[0][lane] + sums[1][lane]) + (sums[2][lane] + sums[3][lane]);
+            float *const all = ref, *const inv = inv_s[warp];
+            all[lane] = total;
+            inv[lane] = __frcp_rn(total);
             __syncwarp();
             if (ok) ok = mbar_wait_warp(o_done + 3, (n - 1) & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -308,7 +336,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) sparse_mla_tc_kernel(const __gr
                 const int at = c * 128 + (warp & 3) * 32 + (lane & ~1);
 #pragma unroll
                 for (int e = 0; e < 32; e += 2) {  // neighbours swap, so that each stores two columns of one head
-                    const float x = o[e] / fix[e], y = o[e + 1] / fix[e + 1];  // the contract divides (no reciprocal)
+                    const float x = sm_quotient(o[e], all[e], inv[e]), y = sm_quotient(o[e + 1], all[e + 1], inv[e + 1]);
                     const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? x : y, 1);
                     if (ok) *reinterpret_cast<uint32_t*>(out + (e + (lane & 1)) * SM_L + at) = (lane & 1) ? pack_bf16(got, y) : pack_bf16(x, got);
                 }
