@@ -105,7 +105,10 @@ __device__ __forceinline__ void load_route_ids(const int* ids, int routes, int E
 
 // grid (pieces of 8 expert channels, routes): the CTA of a group's first route computes the group, 8 gate rows and their 8 up rows, K split
 // over its warps.
-__global__ void __launch_bounds__(MR_THREADS, 2)
+// Two chunks in flight a warp and three CTAs per SM: most of a CTA's time that is not loads is its start (ids, groups) and its sum, which the others cover.  With
+// four chunks and two CTAs (as for the second half, whose CTAs go through all groups: 52 us, with two chunks 56) 122 -> 110 us for eight rows of the top 4 of
+// 64 experts, [2 x 1536 x 4096]; 67 -> 63, 38.2 -> 36.1, 21.3 -> 19.9 for four, two and one.  The weights asked for in L2 by the CTA's first thread: 120.
+__global__ void __launch_bounds__(MR_THREADS, 3)
 expert_glu_mma_kernel(const bf16* __restrict__ x, int64_t xs, int rows, int top, const int* __restrict__ ids, const float* __restrict__ weights,
                       const bf16* __restrict__ gate_up, int E, int F, int K, int kind, bf16* __restrict__ act, uint32_t* status) {
     GLMB_PDL_PROLOGUE();
@@ -122,7 +125,7 @@ expert_glu_mma_kernel(const bf16* __restrict__ x, int64_t xs, int rows, int top,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, n = blockIdx.x * 8;
     const bf16* w = gate_up + ((int64_t)e * 2 * F + n + g) * K;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
-    skinny_mma_span<4>(w, w + (int64_t)F * K, member_s[g] >= 0 ? x + (int64_t)g * xs : nullptr, K, warp, lane & 3, c);
+    skinny_mma_span<2>(w, w + (int64_t)F * K, member_s[g] >= 0 ? x + (int64_t)g * xs : nullptr, K, warp, lane & 3, c);
     skm_store_fragment(red[warp], c, lane);
     __syncthreads();
     const int r = threadIdx.x >> 3, j = threadIdx.x & 7;
