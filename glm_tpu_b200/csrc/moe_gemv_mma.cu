@@ -24,11 +24,39 @@
 #define MM_THREADS (32 * MM_WARPS)
 #define MM_ROWS 16  // output rows per CTA
 
+// A route per tile: routes of the same expert, eight at a time, form a group, and the CTAs of its first route compute all of it, as the columns of the
+// instruction.  Whether route p is the first of its group; members[i]: its i-th route, -1 past the last.  Every warp for itself, so that nobody waits.
+__device__ __forceinline__ bool mm_group(const int* experts, int routes, int p, int lane, int* members) {
+    const int e = experts[p];
+    if (lane < 8) members[lane] = -1;
+    __syncwarp();
+    int seen = 0, first = 0;  // routes of the expert so far, and ahead of p
+    for (int base = 0; base < routes; base += 32) {
+        const bool same = base + lane < routes && experts[base + lane] == e;
+        const unsigned votes = __ballot_sync(0xffffffffu, same);
+        if (p >> 5 == base >> 5) {
+            first = seen + __popc(votes & ((1u << (p & 31)) - 1));
+            if (first & 7) return false;
+        }
+        const int place = seen + __popc(votes & ((1u << lane) - 1)) - first;
+        if (same && base + lane >= p && place < 8) members[place] = base + lane;
+        seen += __popc(votes);
+    }
+    __syncwarp();
+    return true;
+}
+
 // act[p][n] = bf16( silu(bf16(x_p . wg[e][n])) * bf16(x_p . wu[e][n]) ) for the routes p of tile t.  H % 64 == 0, I % 16 == 0.
 // MM_DEPTH: chunks of a warp whose loads are in flight together (4 for grids of up to two CTAs per SM, where DRAM latency is the
 // bound; 1 for large grids, where the registers of a deep pipeline would cost resident CTAs).
-template <int RT, int MM_DEPTH>
-__global__ void __launch_bounds__(MM_THREADS)
+// GROUP: a route per tile in a large grid (a decode step on one GPU), an expert read once for up to eight of its routes.  Bound by latency, and its rate by the
+// registers that the compiler gives it: told to fit four CTAs in an SM (the second half: five) it spends them on loads ahead of the decode.  Eight distinct
+// experts of [2 x 2048 x 6144] and back, in a step: 52.7 + 27.6 -> 43.6 + 25.0 us; three CTAs 52 + 28, five 45.2 + 24.4; two chunks in flight 50 + 27; a
+// multiplication for two codes (four CTAs) 55.7 + 25.8.  Two, four and eight chats 97.9 + 51.1, 177 + 98, 346 + 194 -> 75.4 + 46.3, 133 + 86, 238 + 166 us; a
+// kernel that kept the weights of a persistent CTA's next items in flight with cp.async: 94 + 55, 170 + 97, 312 + 181 with experts that all differ (here 78 +
+// 51, 143 + 92, 272 + 174).  The groups found with barriers of the CTA: 78.7 + 48.1, 140 + 91, 256 + 172.
+template <int RT, int MM_DEPTH, bool GROUP = false>
+__global__ void __launch_bounds__(MM_THREADS, GROUP ? 4 : 0)
 moe_gateup_fp8_mma_kernel(const bf16* __restrict__ x, int64_t xs, int top_k, const int* __restrict__ tile_expert,
                           const int* __restrict__ tile_routes, const int* __restrict__ n_tiles, const uint8_t* __restrict__ wg,
                           const uint8_t* __restrict__ wu, const float* __restrict__ sg, const float* __restrict__ su, int expert_base,
@@ -40,9 +68,12 @@ moe_gateup_fp8_mma_kernel(const bf16* __restrict__ x, int64_t xs, int top_k, con
     const int e = tile_expert[tile] - expert_base;
     if (e < 0 || e >= experts_local) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    __shared__ int members_s[MM_WARPS][8];
+    int* const members = members_s[warp];
+    if (GROUP && !mm_group(tile_expert, gridDim.y, tile, lane, members)) return;
     const int n0 = blockIdx.x * MM_ROWS;
     // activation row of this lane's column g
-    const int route = g < RT ? (tile_routes ? tile_routes[tile * RT + g] : (g == 0 ? tile : -1)) : -1;
+    const int route = GROUP ? members[g] : g < RT ? (tile_routes ? tile_routes[tile * RT + g] : (g == 0 ? tile : -1)) : -1;
     const bf16* xr = x + (int64_t)(route >= 0 ? route / top_k : 0) * xs;
     const int kb = (H + 127) >> 7;
     const uint8_t* wg_lo = wg + ((int64_t)e * I + n0 + g) * H;
@@ -83,9 +114,9 @@ moe_gateup_fp8_mma_kernel(const bf16* __restrict__ x, int64_t xs, int top_k, con
     red[warp][1][g][2 * t] = acc_u[0]; red[warp][1][g][2 * t + 1] = acc_u[1];
     red[warp][1][g + 8][2 * t] = acc_u[2]; red[warp][1][g + 8][2 * t + 1] = acc_u[3];
     __syncthreads();
-    if (threadIdx.x < MM_ROWS * RT) {
+    if (threadIdx.x < MM_ROWS * (GROUP ? 8 : RT)) {
         const int n = threadIdx.x % MM_ROWS, col = threadIdx.x / MM_ROWS;
-        const int p = tile_routes ? tile_routes[tile * RT + col] : (col == 0 ? tile : -1);
+        const int p = GROUP ? members[col] : tile_routes ? tile_routes[tile * RT + col] : (col == 0 ? tile : -1);
         if (p >= 0 && n0 + n < I) {
             float gs = 0.f, us = 0.f;
 #pragma unroll
@@ -97,8 +128,8 @@ moe_gateup_fp8_mma_kernel(const bf16* __restrict__ x, int64_t xs, int top_k, con
 }
 
 // dw[p][n] = bf16( bf16(act[p] . wd[e][n]) * bf16(route_weight[p]) ).  I % 64 == 0, H % 16 == 0.
-template <int RT, int MM_DEPTH>
-__global__ void __launch_bounds__(MM_THREADS)
+template <int RT, int MM_DEPTH, bool GROUP = false>
+__global__ void __launch_bounds__(MM_THREADS, GROUP ? 5 : 0)
 moe_down_fp8_mma_kernel(const bf16* __restrict__ act, const float* __restrict__ route_weight, const int* __restrict__ tile_expert,
                         const int* __restrict__ tile_routes, const int* __restrict__ n_tiles, const uint8_t* __restrict__ wd,
                         const float* __restrict__ sd, int expert_base, int experts_local, int I, int H, bf16* __restrict__ dw) {
@@ -109,8 +140,11 @@ moe_down_fp8_mma_kernel(const bf16* __restrict__ act, const float* __restrict__ 
     const int e = tile_expert[tile] - expert_base;
     if (e < 0 || e >= experts_local) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    __shared__ int members_s[MM_WARPS][8];
+    int* const members = members_s[warp];
+    if (GROUP && !mm_group(tile_expert, gridDim.y, tile, lane, members)) return;
     const int n0 = blockIdx.x * MM_ROWS;
-    const int route = g < RT ? (tile_routes ? tile_routes[tile * RT + g] : (g == 0 ? tile : -1)) : -1;
+    const int route = GROUP ? members[g] : g < RT ? (tile_routes ? tile_routes[tile * RT + g] : (g == 0 ? tile : -1)) : -1;
     const bf16* xr = act + (int64_t)(route >= 0 ? route : 0) * I;
     const int kb = (I + 127) >> 7;
     const uint8_t* w_lo = wd + ((int64_t)e * H + n0 + g) * I;
@@ -139,9 +173,9 @@ moe_down_fp8_mma_kernel(const bf16* __restrict__ act, const float* __restrict__ 
     red[warp][g][2 * t] = acc[0]; red[warp][g][2 * t + 1] = acc[1];
     red[warp][g + 8][2 * t] = acc[2]; red[warp][g + 8][2 * t + 1] = acc[3];
     __syncthreads();
-    if (threadIdx.x < MM_ROWS * RT) {
+    if (threadIdx.x < MM_ROWS * (GROUP ? 8 : RT)) {
         const int n = threadIdx.x % MM_ROWS, col = threadIdx.x / MM_ROWS;
-        const int p = tile_routes ? tile_routes[tile * RT + col] : (col == 0 ? tile : -1);
+        const int p = GROUP ? members[col] : tile_routes ? tile_routes[tile * RT + col] : (col == 0 ? tile : -1);
         if (p >= 0 && n0 + n < H) {
             float s = 0.f;
 #pragma unroll
@@ -306,10 +340,10 @@ int glmb_launch_moe_gateup_mma(const void* x, int64_t xs, int top_k, const int* 
                                int experts_local, int I, int H, void* act, cudaStream_t stream) {
     dim3 grid(ceil_div(I, MM_ROWS), tiles);
     const long live = live_ctas(grid.x, tiles, experts_local);
-#define CALL(RT_, D_)                                                                                                                      \
-    GLMB_LAUNCH((moe_gateup_fp8_mma_kernel<RT_, D_>), grid, MM_THREADS, 0, stream, (const bf16*)x, xs, top_k, tile_expert, tile_routes, n_tiles, \
+#define CALL(RT_, ...)                                                                                                                      \
+    GLMB_LAUNCH((moe_gateup_fp8_mma_kernel<RT_, __VA_ARGS__>), grid, MM_THREADS, 0, stream, (const bf16*)x, xs, top_k, tile_expert, tile_routes, n_tiles, \
                 (const uint8_t*)wg, (const uint8_t*)wu, sg, su, expert_base, experts_local, I, H, (bf16*)act)
-    if (rt == 1) { if (live <= 2 * 148) CALL(1, 4); else if (live <= 4 * 148) CALL(1, 2); else CALL(1, 1); }
+    if (rt == 1) { if (live <= 2 * 148) CALL(1, 4); else if (live <= 4 * 148) CALL(1, 2); else if (!tile_routes && !n_tiles) CALL(1, 1, true); else CALL(1, 1); }
     else CALL(8, 1);
 #undef CALL
     return (int)cudaGetLastError();
@@ -320,10 +354,10 @@ int glmb_launch_moe_down_mma(const void* act, const float* route_weight, const i
                              cudaStream_t stream) {
     dim3 grid(ceil_div(H, MM_ROWS), tiles);
     const long live = live_ctas(grid.x, tiles, experts_local);
-#define CALL(RT_, D_)                                                                                                                        \
-    GLMB_LAUNCH((moe_down_fp8_mma_kernel<RT_, D_>), grid, MM_THREADS, 0, stream, (const bf16*)act, route_weight, tile_expert, tile_routes, n_tiles, \
+#define CALL(RT_, ...)                                                                                                                        \
+    GLMB_LAUNCH((moe_down_fp8_mma_kernel<RT_, __VA_ARGS__>), grid, MM_THREADS, 0, stream, (const bf16*)act, route_weight, tile_expert, tile_routes, n_tiles, \
                 (const uint8_t*)wd, sd, expert_base, experts_local, I, H, (bf16*)dw)
-    if (rt == 1) { if (live <= 2 * 148) CALL(1, 4); else if (live <= 4 * 148) CALL(1, 2); else CALL(1, 1); }
+    if (rt == 1) { if (live <= 2 * 148) CALL(1, 4); else if (live <= 4 * 148) CALL(1, 2); else if (!tile_routes && !n_tiles) CALL(1, 1, true); else CALL(1, 1); }
     else if (tile_routes && I <= 512) {  // a short K: one warp per 16 output rows
         GLMB_LAUNCH(moe_down_fp8_mma_shortk_kernel<8>, dim3(ceil_div(H, MM_ROWS * MM_WARPS), tiles), MM_THREADS, 0, stream, (const bf16*)act,
                     route_weight, tile_expert, tile_routes, n_tiles, (const uint8_t*)wd, sd, expert_base, experts_local, I, H, (bf16*)dw);

@@ -1,4 +1,4 @@
-"""Decode experts streamed once for the routes that chose them: the bits of the kernels with a CTA per route (B200 only)."""
+"""Decode experts read once for the routes that chose them: the bits of the kernels with a CTA per route (B200 only)."""
 
 import pytest
 import torch
@@ -12,7 +12,7 @@ DEV = "cuda:0"
 @pytest.mark.parametrize("rows,tk,E,ebase,el,H,I,same", [
     (4, 8, 64, 0, 64, 6144, 2048, False), (8, 8, 16, 0, 16, 1088, 1040, False), (5, 8, 4, 0, 4, 448, 2064, True), (8, 6, 32, 8, 16, 960, 4096, False),
 ])
-def test_streamed_experts_have_the_bits_of_a_cta_per_route(native_lib, rows, tk, E, ebase, el, H, I, same):
+def test_grouped_routes_have_the_bits_of_a_cta_per_route(native_lib, rows, tk, E, ebase, el, H, I, same):
     n = native_lib
     gen = torch.Generator(device=DEV).manual_seed(rows * tk + H)
     codes = lambda *s: torch.randint(0, 256, s, dtype=torch.uint8, device=DEV, generator=gen).bitwise_and_(0xBF)  # noqa: E731  (no NaN)
