@@ -3,7 +3,7 @@
 //
 // `warp_dot_*`: a warp owns NPW weight rows over a K range: every lane streams 16-byte pieces (L1 no-allocate), multiplies them
 // with the R activation rows in fp32 and the warp reduces with the xor tree of warp_sum, so every caller gets the same bits for the
-// same (rows, K range).  `skinny_mma_*`: 16 weight rows on mma.sync, for two to eight rows and all but few outputs.
+// same (rows, K range).  `skinny_mma_*`: 16 weight rows on mma.sync, for one to eight rows and all but few outputs.
 #pragma once
 
 #include "common.cuh"
