@@ -71,8 +71,9 @@ __device__ __forceinline__ float sm_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// a / b, correctly rounded (the contract divides), of y = the rounded 1 / b: a quotient and one correction by its remainder (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000", theorem 8.5), without the branch of a division.  Infinities keep the first quotient.
+// a / b (the contract divides) of y = the rounded 1 / b: a quotient and one correction by its remainder (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990), without the branch of a division.  Rounded correctly where the first quotient is within an ulp of a / b, else at
+// most the neighbour, 2^-23, of which bf16 keeps 2^-8.  Infinities keep the first quotient.
 __device__ __forceinline__ float sm_quotient(float a, float b, float y) {
     const float q = a * y, exact = fmaf(fmaf(-q, b, a), y, q);
     return exact == exact ? exact : q;
