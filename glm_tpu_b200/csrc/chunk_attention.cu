@@ -229,11 +229,12 @@ __global__ void __launch_bounds__(CP_THREADS) chunk_attn_prefill_kernel(ChunkAtt
 
 // ---------------------------------------------------------------------------------------------------
 #define CD_HEADS 16
+#define CD_SPLITS_OF_TWO 4  // of the form with two parts to a CTA
 // A tile is 16 keys per warp: WARPS * 16 keys, in 64-column boxes of 128-byte rows (128-byte swizzle).
 
 static inline int cd_boxes(int padded) { return (padded + 63) / 64; }
-static inline size_t chunk_decode_smem(int dk, int dv, int stages, int warps) {
-    const size_t tiles = (size_t)stages * (cd_boxes(dk) + cd_boxes(dv)) * warps * 16 * 128, merge = (size_t)warps * CD_HEADS * dv * 4;
+static inline size_t chunk_decode_smem(int dk, int dv, int stages, int warps, int parts) {
+    const size_t tiles = (size_t)stages * (cd_boxes(dk) + cd_boxes(dv)) * warps * 16 * 128, merge = (size_t)parts * warps * CD_HEADS * dv * 4;
     return 1024 + (tiles > merge ? tiles : merge) + (size_t)CD_HEADS * (dk + 8) * 2;
 }
 
@@ -246,20 +247,23 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {  // 8 x 8 matr
 // grid (splits, key heads x blocks of 16 query heads, rows), cluster (splits, 1, 1).
 // A warp's 16 keys are the M of both products (scores: keys x heads; output: value columns x heads), the query heads the N (NT tiles of 8):
 // with the handful of query heads that share a key head, few multiplications are spent on padding.
-template <int DV, int WARPS, int NT>
-__global__ void __launch_bounds__(WARPS * 32)
+// PARTS: a CTA's tiles form so many parts of the keys (every PARTS-th tile is of the same one), which it goes through one after another and whose sums meet as
+// if each had a CTA of its own.  Registers: one CTA an SM may have them all (<128, 8, 2> spilled at the compiler's own choice: 59.8 -> 43.0 us for 8,000 keys of eight
+// key heads with ten query heads each), the others share it with a second one.
+template <int DV, int WARPS, int NT, int PARTS>
+__global__ void __launch_bounds__(WARPS * 32, DV == 128 && WARPS == 8 ? 1 : 2)
 chunk_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, ChunkAttnArgs a, int stages) {
     constexpr int KEYS = WARPS * 16, BOX = KEYS * 128, HEADS = NT * 8;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ unsigned char smem_raw[];
-    __shared__ float ml_s[WARPS][HEADS][2];  // (maximum, sum) per warp
-    __shared__ __align__(8) float cta_ml[HEADS][2];
+    __shared__ float ml_s[PARTS][WARPS][HEADS][2];  // (maximum, sum) per warp
+    __shared__ __align__(8) float cta_ml[PARTS][HEADS][2];
     __shared__ __align__(8) uint64_t full_bar[4];
     const int dk = a.dimp, dv = a.vdimp, KP = dk + 8;
     const int kboxes = (dk + 63) / 64, vboxes = (dv + 63) / 64;
     unsigned char* tiles_s = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const size_t stage_bytes = (size_t)(kboxes + vboxes) * BOX;
-    const size_t tile_area = stages * stage_bytes, merge_area = (size_t)WARPS * HEADS * dv * 4;
+    const size_t tile_area = stages * stage_bytes, merge_area = (size_t)PARTS * WARPS * HEADS * dv * 4;
     bf16* q_s = reinterpret_cast<bf16*>(tiles_s + (tile_area > merge_area ? tile_area : merge_area));
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) mbar_init(full_bar + s, 1);
@@ -270,17 +274,20 @@ chunk_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const int per = a.H / a.G, head_blocks = (per + CD_HEADS - 1) / CD_HEADS;
     const int group = blockIdx.y / head_blocks, h0 = group * per + (blockIdx.y % head_blocks) * CD_HEADS;
     const int heads = min(CD_HEADS, group * per + per - h0);
-    const int row = blockIdx.z, split = blockIdx.x, splits = gridDim.x;
+    const int row = blockIdx.z, split = blockIdx.x, splits = PARTS > 1 ? CD_SPLITS_OF_TWO : gridDim.x;
     const bool active = !a.row_active || a.row_active[row] != 0;
     const int pos = ca_pos(a, row), lane_id = ca_lane(a, row);
     const int keys = active ? pos % a.chunk + 1 : 0;  // slots 0 .. keys - 1 of the lane's ring
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mr = lane & 7, mi = lane >> 3;
     const int tiles = (keys + KEYS - 1) / KEYS, mine = tiles > split ? (tiles - split - 1) / splits + 1 : 0;  // tiles split, split + splits, ..
 
+    const int in_first = (mine + PARTS - 1) / PARTS;
+    static_assert(PARTS <= 2, "order of the tiles");
+    auto tile_at = [&](int i) { return split + (PARTS == 1 ? i : i < in_first ? 2 * i : 2 * (i - in_first) + 1) * splits; };
     auto load_tile = [&](int i) {  // the i-th tile of this CTA, by one thread
         unsigned char* dst = tiles_s + (size_t)(i % stages) * stage_bytes;
         uint64_t* bar = full_bar + i % stages;
-        const int y = lane_id * a.ring + (split + i * splits) * KEYS;
+        const int y = lane_id * a.ring + tile_at(i) * KEYS;
         mbar_expect_tx(bar, (uint32_t)stage_bytes);
         for (int b = 0; b < kboxes; ++b) tma_load_2d(dst + b * BOX, &map_k, bar, group * dk + b * 64, y);
         for (int b = 0; b < vboxes; ++b) tma_load_2d(dst + (kboxes + b) * BOX, &map_v, bar, group * dv + b * 64, y);
@@ -298,15 +305,6 @@ chunk_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     __syncthreads();
 
     const float scale2 = a.scale * CA_LOG2E;
-    float m[NT][2], l[NT][2];  // of heads 8 n + 2 t4 + e, equal on the lanes that share t4 (m) or this lane's keys (l)
-    float o[DV / 16][NT][4];   // value columns 16 j + g, + 8; heads 8 n + 2 t4, + 1
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        m[n][0] = m[n][1] = -INFINITY;
-        l[n][0] = l[n][1] = 0.f;
-#pragma unroll
-        for (int j = 0; j < DV / 16; ++j) o[j][n][0] = o[j][n][1] = o[j][n][2] = o[j][n][3] = 0.f;
-    }
     // this lane's rows of a key / value fragment and its 16-byte pieces of a 128-byte row, as they lie swizzled
     const int k_row = (mr + 8 * (mi & 1)) * 128, v_row = (mr + 8 * (mi >> 1)) * 128;
     int k_col[4], v_col[4];
@@ -328,154 +326,195 @@ chunk_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             if (c * 16 < dk) load_q(qf[c], c * 16);
     }
     bool ok = true;
-    for (int i = 0; i < mine; ++i) {
-        const int stage = i % stages, slot0 = (split + i * splits) * KEYS;
-        if (ok && !mbar_wait(full_bar + stage, (i / stages) & 1)) {
-            if (lane == 0) raise_status(a.status, GLMB_STATUS_WAIT_TIMEOUT);
-            ok = false;  // no more work for this warp, but it still meets the others at their barriers
-        }
-        unsigned char* kt = tiles_s + (size_t)stage * stage_bytes;
-        unsigned char* vt = kt + kboxes * BOX;
-        const int w0 = warp * 16, left = ok ? keys - slot0 - w0 : 0;  // this warp's keys of the tile, how many of them exist
-        if (left > 0 && left < 16) {  // values past the last key meet zero weights: they must not be infinite or NaN
-            for (int x = lane; x < (16 - left) * vboxes * 8; x += 32)
-                *reinterpret_cast<uint4*>(vt + (x % (vboxes * 8) >> 3) * BOX + (w0 + left + x / (vboxes * 8)) * 128 + (x & 7) * 16) = make_uint4(0, 0, 0, 0);
-            __syncwarp();
-        }
-        if (left > 0) {
-            float s[NT][4];  // keys g, g + 8; heads 8 n + 2 t4, + 1
-#pragma unroll
-            for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-            const unsigned char* kb = kt + w0 * 128 + k_row;
-            auto step = [&](const uint32_t (&f)[2 * NT], const unsigned char* at) {
-                uint32_t kf[4];
-                ldmatrix_x4(kf, at);
-#pragma unroll
-                for (int n = 0; n < NT; ++n) mma_bf16_16816(s[n], kf, f[2 * n], f[2 * n + 1]);
-            };
-            if constexpr (QSTEPS > 1) {
-#pragma unroll
-                for (int c = 0; c < QSTEPS; ++c)
-                    if (c * 16 < dk) step(qf[c], kb + (c >> 2) * BOX + k_col[c & 3]);
-            } else {
-                for (int k0 = 0; k0 < dk; k0 += 64, kb += BOX)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (k0 + c * 16 < dk) {
-                            load_q(qf[0], k0 + c * 16);
-                            step(qf[0], kb + k_col[c]);
-                        }
-            }
-            uint32_t hi[NT][2], lw[NT][2];  // weights as the second operand: keys x heads
-            float fix[NT][2];
+    float m[NT][2], l[NT][2];  // of heads 8 n + 2 t4 + e, equal on the lanes that share t4 (m) or this lane's keys (l)
+    float o[DV / 16][NT][4];   // value columns 16 j + g, + 8; heads 8 n + 2 t4, + 1
+    float first_m[NT][2], first_l[NT][2], first_o[DV / 16][NT][4];  // of the first of two parts, while the second is gone through
+#pragma unroll 1
+    for (int part = 0, i = 0; part < PARTS; ++part) {
+        if (PARTS > 1 && part > 0) {
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
+                first_m[n][0] = m[n][0]; first_m[n][1] = m[n][1];
+                first_l[n][0] = l[n][0]; first_l[n][1] = l[n][1];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[n][e] = g + 8 * (e >> 1) >= left ? -INFINITY : s[n][e] * scale2;
+                for (int j = 0; j < DV / 16; ++j)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float top = fmaxf(s[n][e], s[n][2 + e]);
-                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
-                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
-                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
-                    top = fmaxf(top, m[n][e]);  // at least one key exists: finite
-                    fix[n][e] = exp2f(m[n][e] - top);
-                    m[n][e] = top;
-                    s[n][e] = exp2f(s[n][e] - top);
-                    s[n][2 + e] = exp2f(s[n][2 + e] - top);
-                    l[n][e] = l[n][e] * fix[n][e] + s[n][e] + s[n][2 + e];
-                }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    uint32_t x, y;
-                    ca_split(s[n][2 * e], s[n][2 * e + 1], x, y);
-                    hi[n][e] = movmatrix_trans(x);
-                    lw[n][e] = movmatrix_trans(y);
-                }
+                    for (int e = 0; e < 4; ++e) first_o[j][n][e] = o[j][n][e];
             }
-            bool moved = false;
+        }
 #pragma unroll
-            for (int n = 0; n < NT; ++n) moved |= fix[n][0] != 1.f || fix[n][1] != 1.f;
-            moved = __any_sync(0xffffffffu, moved);
+        for (int n = 0; n < NT; ++n) {
+            m[n][0] = m[n][1] = -INFINITY;
+            l[n][0] = l[n][1] = 0.f;
 #pragma unroll
-            for (int j = 0; j < DV / 16; ++j)
-                if (j * 16 < dv) {
-                    uint32_t vf[4];
-                    ldmatrix_x4_trans(vf, vt + (j >> 2) * BOX + w0 * 128 + v_row + v_col[j & 3]);
+            for (int j = 0; j < DV / 16; ++j) o[j][n][0] = o[j][n][1] = o[j][n][2] = o[j][n][3] = 0.f;
+        }
+        for (const int end = part == PARTS - 1 ? mine : in_first; i < end; ++i) {
+            const int stage = i % stages, slot0 = tile_at(i) * KEYS;
+            if (ok && !mbar_wait(full_bar + stage, (i / stages) & 1)) {
+                if (lane == 0) raise_status(a.status, GLMB_STATUS_WAIT_TIMEOUT);
+                ok = false;  // no more work for this warp, but it still meets the others at their barriers
+            }
+            unsigned char* kt = tiles_s + (size_t)stage * stage_bytes;
+            unsigned char* vt = kt + kboxes * BOX;
+            const int w0 = warp * 16, left = ok ? keys - slot0 - w0 : 0;  // this warp's keys of the tile, how many of them exist
+            if (left > 0 && left < 16) {  // values past the last key meet zero weights: they must not be infinite or NaN
+                for (int x = lane; x < (16 - left) * vboxes * 8; x += 32)
+                    *reinterpret_cast<uint4*>(vt + (x % (vboxes * 8) >> 3) * BOX + (w0 + left + x / (vboxes * 8)) * 128 + (x & 7) * 16) = make_uint4(0, 0, 0, 0);
+                if constexpr (PARTS > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stage may be filled again, for the next part
+                __syncwarp();
+            }
+            if (left > 0) {
+                float s[NT][4];  // keys g, g + 8; heads 8 n + 2 t4, + 1
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) {
-                        if (moved) { o[j][n][0] *= fix[n][0]; o[j][n][1] *= fix[n][1]; o[j][n][2] *= fix[n][0]; o[j][n][3] *= fix[n][1]; }
-                        mma_bf16_16816(o[j][n], vf, hi[n][0], hi[n][1]);
-                        mma_bf16_16816(o[j][n], vf, lw[n][0], lw[n][1]);
+                for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+                const unsigned char* kb = kt + w0 * 128 + k_row;
+                auto step = [&](const uint32_t (&f)[2 * NT], const unsigned char* at) {
+                    uint32_t kf[4];
+                    ldmatrix_x4(kf, at);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) mma_bf16_16816(s[n], kf, f[2 * n], f[2 * n + 1]);
+                };
+                if constexpr (QSTEPS > 1) {
+#pragma unroll
+                    for (int c = 0; c < QSTEPS; ++c)
+                        if (c * 16 < dk) step(qf[c], kb + (c >> 2) * BOX + k_col[c & 3]);
+                } else {
+                    for (int k0 = 0; k0 < dk; k0 += 64, kb += BOX)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (k0 + c * 16 < dk) {
+                                load_q(qf[0], k0 + c * 16);
+                                step(qf[0], kb + k_col[c]);
+                            }
+                }
+                uint32_t hi[NT][2], lw[NT][2];  // weights as the second operand: keys x heads
+                float fix[NT][2];
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[n][e] = g + 8 * (e >> 1) >= left ? -INFINITY : s[n][e] * scale2;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float top = fmaxf(s[n][e], s[n][2 + e]);
+                        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+                        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+                        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+                        top = fmaxf(top, m[n][e]);  // at least one key exists: finite
+                        fix[n][e] = exp2f(m[n][e] - top);
+                        m[n][e] = top;
+                        s[n][e] = exp2f(s[n][e] - top);
+                        s[n][2 + e] = exp2f(s[n][2 + e] - top);
+                        l[n][e] = l[n][e] * fix[n][e] + s[n][e] + s[n][2 + e];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        uint32_t x, y;
+                        ca_split(s[n][2 * e], s[n][2 * e + 1], x, y);
+                        hi[n][e] = movmatrix_trans(x);
+                        lw[n][e] = movmatrix_trans(y);
                     }
                 }
-        }
-        if (i + stages < mine) {  // every warp has read the stage: fill it again
-            __syncthreads();
-            if (threadIdx.x == 0) load_tile(i + stages);
+                bool moved = false;
+#pragma unroll
+                for (int n = 0; n < NT; ++n) moved |= fix[n][0] != 1.f || fix[n][1] != 1.f;
+                moved = __any_sync(0xffffffffu, moved);
+#pragma unroll
+                for (int j = 0; j < DV / 16; ++j)
+                    if (j * 16 < dv) {
+                        uint32_t vf[4];
+                        ldmatrix_x4_trans(vf, vt + (j >> 2) * BOX + w0 * 128 + v_row + v_col[j & 3]);
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            if (moved) { o[j][n][0] *= fix[n][0]; o[j][n][1] *= fix[n][1]; o[j][n][2] *= fix[n][0]; o[j][n][3] *= fix[n][1]; }
+                            mma_bf16_16816(o[j][n], vf, hi[n][0], hi[n][1]);
+                            mma_bf16_16816(o[j][n], vf, lw[n][0], lw[n][1]);
+                        }
+                    }
+            }
+            if (i + stages < mine) {  // every warp has read the stage: fill it again
+                __syncthreads();
+                if (threadIdx.x == 0) load_tile(i + stages);
+            }
         }
     }
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float sum = l[n][e];
-            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-            if (g == 0) { ml_s[warp][n * 8 + 2 * t4 + e][0] = m[n][e]; ml_s[warp][n * 8 + 2 * t4 + e][1] = sum; }
-        }
     __syncthreads();  // every warp has left the tiles: the merge area takes their place
-    float* o_s = reinterpret_cast<float*>(tiles_s);  // [warp][head][dv]
+    float* o_s = reinterpret_cast<float*>(tiles_s);  // [part][warp][head][dv]
+    const int part_area = WARPS * HEADS * dv;
+    auto hand_in = [&](int part, float (&m)[NT][2], float (&l)[NT][2], float (&o)[DV / 16][NT][4]) {
 #pragma unroll
-    for (int j = 0; j < DV / 16; ++j)
-        if (j * 16 < dv)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+            for (int e = 0; e < 2; ++e) {
+                float sum = l[n][e];
+                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+                if (g == 0) { ml_s[part][warp][n * 8 + 2 * t4 + e][0] = m[n][e]; ml_s[part][warp][n * 8 + 2 * t4 + e][1] = sum; }
+            }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) o_s[((size_t)warp * HEADS + n * 8 + 2 * t4 + (e & 1)) * dv + j * 16 + g + 8 * (e >> 1)] = o[j][n][e];
+        for (int j = 0; j < DV / 16; ++j)
+            if (j * 16 < dv)
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        o_s[part * part_area + (warp * HEADS + n * 8 + 2 * t4 + (e & 1)) * dv + j * 16 + g + 8 * (e >> 1)] = o[j][n][e];
+    };
+    if constexpr (PARTS > 1) hand_in(0, first_m, first_l, first_o);
+    hand_in(PARTS - 1, m, l, o);
     __syncthreads();
-    // ---- warps of the CTA into warp 0's area ------------------------------------------------------------
-    if (threadIdx.x < HEADS) {
+    // ---- warps of the CTA into warp 0's area, part by part ----------------------------------------------
+    if (threadIdx.x < PARTS * HEADS) {
+        const int part = threadIdx.x / HEADS, h = threadIdx.x % HEADS;
+        float (*ml)[HEADS][2] = ml_s[part];
         float top = -INFINITY, sum = 0.f;
-        for (int w = 0; w < WARPS; ++w) top = fmaxf(top, ml_s[w][threadIdx.x][0]);
-        for (int w = 0; w < WARPS; ++w)
-            if (ml_s[w][threadIdx.x][0] != -INFINITY) sum += ml_s[w][threadIdx.x][1] * exp2f(ml_s[w][threadIdx.x][0] - top);
-        cta_ml[threadIdx.x][0] = top;
-        cta_ml[threadIdx.x][1] = sum;
+        for (int w = 0; w < WARPS; ++w) top = fmaxf(top, ml[w][h][0]);
+        for (int w = 0; w < WARPS; ++w) {
+            const float weight = ml[w][h][0] == -INFINITY ? 0.f : exp2f(ml[w][h][0] - top);
+            sum += ml[w][h][1] * weight;
+            ml[w][h][0] = weight;
+        }
+        cta_ml[part][h][0] = top;
+        cta_ml[part][h][1] = sum;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < HEADS * dv; i += WARPS * 32) {
         const int h = i / dv;
-        const float top = cta_ml[h][0];
-        float v = 0.f;
-        for (int w = 0; w < WARPS; ++w)
-            if (ml_s[w][h][0] != -INFINITY) v += o_s[(size_t)w * HEADS * dv + i] * exp2f(ml_s[w][h][0] - top);
-        o_s[i] = v;
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part) {
+            float* o_part = o_s + part * part_area + i;
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) v += o_part[w * HEADS * dv] * ml_s[part][w][h][0];
+            *o_part = v;
+        }
     }
     cluster.sync();
     // ---- CTAs of the cluster: each finishes its share of the outputs, the sink joins here -----------------
-    // First every CTA's (maximum, sum) of every head, all loads at once, then a weight per CTA and head.
-    __shared__ float part_s[16][HEADS][2];
-    for (int i = threadIdx.x; i < splits * HEADS; i += WARPS * 32) {
-        const float2 ml = *reinterpret_cast<const float2*>(cluster.map_shared_rank(&cta_ml[0][0], i / HEADS) + (i % HEADS) * 2);
-        part_s[i / HEADS][i % HEADS][0] = ml.x;
-        part_s[i / HEADS][i % HEADS][1] = ml.y;
+    // First every part's (maximum, sum) of every head, all loads at once, then a weight per part and head.  Part p is part p / splits of CTA p % splits.
+    __shared__ float parts_s[16][HEADS][2];
+    const int parts = splits * PARTS;
+    for (int i = threadIdx.x; i < parts * HEADS; i += WARPS * 32) {
+        const int p = i / HEADS, part = PARTS > 1 && p >= splits;
+        const float2 ml = *reinterpret_cast<const float2*>(cluster.map_shared_rank(&cta_ml[part][0][0], p - part * splits) + (i % HEADS) * 2);
+        parts_s[p][i % HEADS][0] = ml.x;
+        parts_s[p][i % HEADS][1] = ml.y;
     }
     __syncthreads();
     if ((int)threadIdx.x < heads) {
         const int h = threadIdx.x;
         const float sink2 = a.sink ? a.sink[h0 + h] * CA_LOG2E : -INFINITY;
         float top = sink2;
-        for (int p = 0; p < splits; ++p) top = fmaxf(top, part_s[p][h][0]);
+        for (int p = 0; p < parts; ++p) top = fmaxf(top, parts_s[p][h][0]);
         float sum = a.sink ? exp2f(sink2 - top) : 0.f;
-        for (int p = 0; p < splits; ++p) {
-            const float w = part_s[p][h][0] == -INFINITY ? 0.f : exp2f(part_s[p][h][0] - top);
-            sum += part_s[p][h][1] * w;
-            part_s[p][h][0] = w;
+        for (int p = 0; p < parts; ++p) {
+            const float w = parts_s[p][h][0] == -INFINITY ? 0.f : exp2f(parts_s[p][h][0] - top);
+            sum += parts_s[p][h][1] * w;
+            parts_s[p][h][0] = w;
         }
         const float inv = sum > 0.f ? ca_gate<bf16>(a, row, h0 + h) / sum : 0.f;
-        for (int p = 0; p < splits; ++p) part_s[p][h][0] *= inv;
+        for (int p = 0; p < parts; ++p) parts_s[p][h][0] *= inv;
     }
     __syncthreads();
     const int total = heads * a.vdim;
@@ -483,8 +522,10 @@ chunk_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     for (int i = split * WARPS * 32 + threadIdx.x; i < total; i += splits * WARPS * 32) {
         const int h = i / a.vdim, c = i % a.vdim;
         float v = 0.f;
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part)
 #pragma unroll 16
-        for (int p = 0; p < splits; ++p) v = fmaf(cluster.map_shared_rank(o_s, p)[h * dv + c], part_s[p][h][0], v);
+            for (int p = 0; p < splits; ++p) v = fmaf(cluster.map_shared_rank(o_s, p)[part * part_area + h * dv + c], parts_s[part * splits + p][h][0], v);
         out[i] = __float2bfloat16_rn(v);
     }
     cluster.sync();  // nobody leaves while a peer may still read its shared memory
@@ -599,21 +640,35 @@ static int launch_chunk_prefill(const ChunkAttnArgs& a, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
-// Several rows of eight key heads or more: 32 CTAs a row, whatever the number of rows (a row's sums do not depend on it), with rings of 100 KB (head sizes up
-// to 128), so that two CTAs share an SM and all are resident at once.  With rings of 200 KB and eight splits, 256 CTAs (four rows) ran in two
-// waves, and 128 in clusters of eight did not reach every SM: four chats at 1,000 (32 query heads over 8 key heads of 128) 27.0 -> 12.9 us, eight at
-// 3,000 34.4 -> 25.9, two at 3,000 23.8 -> 23.5.  With four key heads half as many CTAs fit one wave up to four rows: three chats at 700 9.7 us there, 10.4 here.
-static bool chunk_decode_many(const ChunkAttnArgs& a) { return a.rows > 1 && a.G * ceil_div(a.H / a.G, CD_HEADS) >= 8; }
+#define CD_RING_ONE (200 * 1024)  // shared memory of a CTA alone on its SM
+#define CD_RING_TWO (104 * 1024)  // ... of two (head sizes above 128: 140 KB, one)
+#define CD_RING_SHALLOW 2048
 
-template <int DV, int WARPS, int NT>
-static int launch_chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
+static int chunk_decode_heads(const ChunkAttnArgs& a) { return a.G * ceil_div(a.H / a.G, CD_HEADS); }
+// Splits (a power of two, at least a tile of the ring each) of a row's `heads`: no more than `ctas` CTAs a row.
+static int chunk_decode_share(const ChunkAttnArgs& a, int warps, int heads, int ctas) {
+    const int tiles = ceil_div(a.ring, warps * 16);
+    int splits = 1;
+    while (splits < 8 && splits * 2 <= tiles && splits * 2 * heads <= ctas) splits *= 2;
+    return splits;
+}
+// As many splits as run at once: clusters of 1, 2, 4, 8 CTAs that a B200 holds (cudaOccupancyMaxActiveClusters), with two CTAs per SM and with one.
+static int chunk_decode_wave(const ChunkAttnArgs& a, int warps, int clusters, bool two) {
+    const int fit[2][4] = {{148, 74, 33, 15}, {296, 148, 71, 33}}, tiles = ceil_div(a.ring, warps * 16);
+    int e = 0;
+    while (e < 3 && (2 << e) <= tiles && clusters <= fit[two][e + 1]) ++e;
+    return 1 << e;
+}
+
+template <int DV, int WARPS, int NT, int PARTS = 1>
+static int launch_chunk_decode(const ChunkAttnArgs& a, int splits, int ring_bytes, cudaStream_t st) {
     static DeviceOnce once;
-    cudaError_t e = chunk_smem_limit(chunk_attn_decode_kernel<DV, WARPS, NT>, once);
+    cudaError_t e = chunk_smem_limit(chunk_attn_decode_kernel<DV, WARPS, NT, PARTS>, once);
     if (e != cudaSuccess) return (int)e;
     static DeviceOnce wide;  // clusters of 16 are beyond the portable size
     const int wide_dev = wide.pending();
     if (wide_dev != DeviceOnce::SET) {
-        e = cudaFuncSetAttribute(chunk_attn_decode_kernel<DV, WARPS, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(chunk_attn_decode_kernel<DV, WARPS, NT, PARTS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
         wide.mark(wide_dev);
     }
@@ -621,19 +676,12 @@ static int launch_chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
     const uint64_t ring_rows = (uint64_t)a.lanes * a.ring;
     if (make_map(&map_k, a.k, ring_rows, (uint64_t)a.G * a.dimp, (uint64_t)a.G * a.dimp, WARPS * 16)) return 3;
     if (make_map(&map_v, a.v, ring_rows, (uint64_t)a.G * a.vdimp, (uint64_t)a.G * a.vdimp, WARPS * 16)) return 3;
-    const int heads = a.G * ceil_div(a.H / a.G, CD_HEADS), tiles = ceil_div(a.ring, WARPS * 16), most = heads * a.rows <= 4 ? 16 : 8;
-    const bool many = chunk_decode_many(a);
-    int stages = 4, splits = 1;
-    while (stages > 2 && chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS) > (many ? 104 : 200) * 1024) --stages;
-    if (many)
-        while (splits < 8 && splits * 2 <= tiles && splits * 2 * heads <= 32) splits *= 2;
-    else  // CTAs per cluster: enough that the grid reaches every SM, at least one tile each.  A cluster of 16 only while few are launched: the
-          // GPU places a handful of them at a time, and eight waited for one another (20 us before the first key, 10 us with eight per cluster).
-        while (splits < most && splits * 2 <= tiles && splits * heads * a.rows < 148) splits *= 2;
+    int stages = 4;
+    while (stages > 2 && chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS, PARTS) > (size_t)ring_bytes) --stages;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(splits, heads, a.rows);
+    cfg.gridDim = dim3(splits, chunk_decode_heads(a), a.rows);
     cfg.blockDim = dim3(WARPS * 32);
-    cfg.dynamicSmemBytes = chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS);
+    cfg.dynamicSmemBytes = chunk_decode_smem(a.dimp, a.vdimp, stages, WARPS, PARTS);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -643,8 +691,38 @@ static int launch_chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, chunk_attn_decode_kernel<DV, WARPS, NT>, map_k, map_v, a, stages);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, chunk_attn_decode_kernel<DV, WARPS, NT, PARTS>, map_k, map_v, a, stages);
     return le != cudaSuccess ? (int)le : (int)cudaGetLastError();
+}
+
+template <int NT>
+static int chunk_decode(const ChunkAttnArgs& a, cudaStream_t st) {
+    const int heads = chunk_decode_heads(a), all = heads * a.rows;
+    const bool dims256 = a.dimp > 128 || a.vdimp > 128, values64 = !dims256 && a.vdimp <= 64;
+    // Several rows of eight key heads or more.  A CTA of four warps takes 1.4 us a tile of 64 keys whatever else its SM does, so the time is that of the longest
+    // CTA: rings of 100 KB, so that two share an SM, and as many splits as run at once.  With rings of 200 KB and eight splits, 256 CTAs ran in two waves.  A
+    // row's sums depend on its parts of the keys, which for 8 - 16 heads are the same for every number of rows: of eight heads 32 CTAs a row on short rings, 64 on
+    // long ones, where from five rows on (a wave holds 33 clusters of eight) a CTA has two parts of them.  More heads on long rings, or more than 16: by the rows.
+    // Us for 8,000 keys of 128, eight key heads, 2, 3, 4, 8 rows: 30.0, 31.9, 32.5, 55.5 (32 CTAs a row: 51.1, 52.8, 53.5, 55.4; eight splits, a CTA an SM: 37.9,
+    // 40.2, 57.9, 64.0), for 1,000: 10.1, 10.9, 11.4, 14.8 (12.1, 12.7, 13.1, 14.7; 17.9, 18.7, 27.1, 22.1); sixteen heads, 8,000 keys: 32.5, 54.2, 54.7, 99.8 (95, 97,
+    // 98, 100; 58, 62, 64, 108).  Two parts cost 0.5 us; in fragments of 16 query heads 10 %, so those keep 32 CTAs a row.  Head sizes of 256, eight heads, 8,000
+    // keys: 79, 80, 80, 159 (eight splits: 92, 94, 140, 169).  Where a wave ends just short (9 heads, 8 rows, 8,000 keys) two waves of twice the splits are 7 % faster.
+    if (a.rows > 1 && heads >= 8) {
+        const bool shallow = a.ring <= CD_RING_SHALLOW;
+        if (dims256) return launch_chunk_decode<256, 4, NT>(a, heads == 8 ? chunk_decode_share(a, 4, 8, 32) : chunk_decode_wave(a, 4, all, false), CD_RING_TWO, st);
+        if (values64) return launch_chunk_decode<64, 8, NT>(a, heads <= 16 ? chunk_decode_share(a, 8, heads, 32) : chunk_decode_wave(a, 8, all, true), CD_RING_TWO, st);
+        if (heads <= 16 && (shallow || (heads == 8 && NT == 2))) return launch_chunk_decode<128, 4, NT>(a, chunk_decode_share(a, 4, heads, 32), CD_RING_TWO, st);
+        if constexpr (NT == 1)
+            if (heads == 8 && a.rows > 4) return launch_chunk_decode<128, 4, NT, 2>(a, CD_SPLITS_OF_TWO, CD_RING_TWO, st);
+        return launch_chunk_decode<128, 4, NT>(a, chunk_decode_wave(a, 4, all, true), CD_RING_TWO, st);
+    }
+    // CTAs per cluster: enough that the grid reaches every SM, at least one tile each.  A cluster of 16 only while few are launched: the
+    // GPU places a handful of them at a time, and eight waited for one another (20 us before the first key, 10 us with eight per cluster).
+    const int warps = dims256 ? 4 : 8, tiles = ceil_div(a.ring, warps * 16), most = all <= 4 ? 16 : 8;
+    int splits = 1;
+    while (splits < most && splits * 2 <= tiles && splits * all < 148) splits *= 2;
+    if (dims256) return launch_chunk_decode<256, 4, NT>(a, splits, CD_RING_ONE, st);
+    return values64 ? launch_chunk_decode<64, 8, NT>(a, splits, CD_RING_ONE, st) : launch_chunk_decode<128, 8, NT>(a, splits, CD_RING_ONE, st);
 }
 
 GLMB_API size_t glmb_chunk_attn_args_sizeof(void) { return sizeof(ChunkAttnArgs); }
@@ -667,12 +745,7 @@ GLMB_API int glmb_chunk_attn_prefill(const ChunkAttnArgs* args, void* stream) {
 GLMB_API int glmb_chunk_attn_decode(const ChunkAttnArgs* args, void* stream) {
     ChunkAttnArgs a = chunk_args(args);
     if (!chunk_args_ok(a) || !a.decode || a.dimp > 256 || a.vdimp > 256) return 1;
-    const bool few = a.H / a.G <= 8;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (a.dimp > 128 || a.vdimp > 128) return few ? launch_chunk_decode<256, 4, 1>(a, st) : launch_chunk_decode<256, 4, 2>(a, st);
-    if (a.vdimp <= 64) return few ? launch_chunk_decode<64, 8, 1>(a, st) : launch_chunk_decode<64, 8, 2>(a, st);
-    if (chunk_decode_many(a)) return few ? launch_chunk_decode<128, 4, 1>(a, st) : launch_chunk_decode<128, 4, 2>(a, st);
-    return few ? launch_chunk_decode<128, 8, 1>(a, st) : launch_chunk_decode<128, 8, 2>(a, st);
+    return a.H / a.G <= 8 ? chunk_decode<1>(a, (cudaStream_t)stream) : chunk_decode<2>(a, (cudaStream_t)stream);
 }
 
 // Any head size (values up to 1024 columns), bf16 or fp32.

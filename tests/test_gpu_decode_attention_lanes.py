@@ -33,3 +33,37 @@ def test_a_rows_bits_do_not_depend_on_the_others(native_lib, H, G, dim):
         results.append(out)
     assert int(status) == 0
     assert torch.equal(results[0], results[2][:2]) and torch.equal(results[1], results[2][:3])
+
+
+# three, four and eight key heads (also with two blocks of query heads in a fragment), sixteen of 64, head sizes of every kernel: a part of the keys per CTA
+# and two, parts of unequal length and without a key
+@pytest.mark.parametrize("H,G,dim", [(12, 3, 128), (16, 4, 64), (32, 8, 128), (80, 8, 128), (32, 8, 64), (16, 16, 64), (32, 8, 256)])
+def test_a_rows_bits_deep_in_a_ring(native_lib, H, G, dim):
+    lanes, ring, positions = 8, 8192, [8000, 63, 5017, 8191, 64, 3000, 511, 1]
+    gen = torch.Generator(device="cuda").manual_seed(G + dim)
+    draw = lambda *s: torch.randn(s, device="cuda", generator=gen).to(torch.bfloat16)  # noqa: E731
+    q, k, v = draw(lanes, H, dim), draw(lanes, ring, G, dim), draw(lanes, ring, G, dim)
+    pos, lane, sink = torch.tensor(positions, dtype=torch.int32, device="cuda"), torch.arange(lanes, dtype=torch.int32, device="cuda"), torch.zeros(H, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def rows_of(rows):
+        out = torch.full((rows, H * dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+        a = single.attention_args(native_lib, q[:rows], k, v, sink, dim**-0.5, out, H, G, dim, dim, status)
+        a.row_pos, a.row_lane, a.row_active = pos.data_ptr(), lane.data_ptr(), None
+        a.rows, a.decode, a.chunk, a.ring, a.capacity, a.lanes = rows, 1, ring, ring, ring, lanes
+        native_lib.chunk_attention(a, False)
+        return out
+
+    all_rows = rows_of(8)
+    for rows in range(2, 8):
+        assert torch.equal(rows_of(rows), all_rows[:rows]), rows
+    assert int(status) == 0
+    for r in (0, 1, 5):
+        n = positions[r] + 1
+        keys, values = (t[r, :n].double().repeat_interleave(H // G, 1) for t in (k, v))
+        score = torch.einsum("hd,jhd->hj", q[r].double(), keys) * dim**-0.5
+        weight = torch.exp(score - score.amax(1, keepdim=True).clamp(min=0))
+        weight = weight / (weight.sum(1, keepdim=True) + torch.exp(-score.amax(1, keepdim=True).clamp(min=0)))  # the sink's score is 0
+        want = torch.einsum("hj,jhd->hd", weight, values).flatten()
+        # products and sums in fp32 (weights as two bf16 pieces), one rounding to bf16: 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
+        assert float((all_rows[r].double() - want).norm() / want.norm()) < 2e-3, r
