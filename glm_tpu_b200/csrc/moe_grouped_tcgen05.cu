@@ -31,8 +31,8 @@
 // (moe_gemv_mma.cu), which decodes an expert again for every eight routes: 60 rows (218 experts) 1,115 + 680 -> 920 + 490 us, 200 rows 1,497 + 933
 // -> 1,131 + 620, 256 rows 1,724 + 1,075 -> 1,160 + 623.  On the way there, 60 rows: the gather in warp 0, between the weights' copies, 1,321 + 682; sixteen
 // decode warps on every step 1,128 + 582; a multiplication per code instead of one for two 976 + 523.
-// Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores (tiles of eight: stores NaN, their entry points
-// have no status word) and still frees its TMEM.
+// Every mbarrier wait is bounded; on a timeout the kernel raises GLMB_STATUS_WAIT_TIMEOUT, skips its stores (tiles of eight: stores NaN, for callers that hand
+// no status word) and still frees its TMEM.
 //
 // Replaces reference `glm_tpu/kernels/fp8_grouped_matmul/panel_kernel.py:31-153` + `layers/moe/routed_experts.py:27-127`
 // (prefill: stable group-by-expert, M32 panels, three FP8 panel matmuls, bf16 SiLU, bf16 route weighting).
@@ -449,7 +449,7 @@ moe_grouped_fp8w_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             if (!done || __any_sync(0xffffffffu, fail)) {
                 fail = 1;
                 if (lane == 0) raise_status(a.status, GLMB_STATUS_WAIT_TIMEOUT);
-                if constexpr (TILES8)  // this form's entry points have no status word: what is missing becomes NaN, which the logits' check finds
+                if constexpr (TILES8)  // a caller may have no status word: what is missing becomes NaN
                     for (; it < items; it += gridDim.x) {
                         const TcTile rest = tile_of(it);
                         for (int r = rest.row0; r < rest.row_end; ++r)
@@ -543,7 +543,7 @@ bool moe_tiles8_takes(const void* x, int64_t x_stride, const void* w0, const voi
 }
 int launch_moe_tiles8(const void* x, int64_t x_stride, int divisor, const int* tile_expert, const int* tile_routes, const int* n_tiles, int tiles,
                       const void* w0, const void* w1, const float* s0, const float* s1, int expert_base, int experts_local, int N, int K, int mode,
-                      const float* route_weight, void* out, cudaStream_t stream) {
+                      const float* route_weight, void* out, uint32_t* status, cudaStream_t stream) {
     CUtensorMap map_w0, map_w1;
     if (make_map_u8(&map_w0, w0, (uint64_t)experts_local * N, (uint64_t)K, (uint64_t)K, 128)) return 3;
     if (make_map_u8(&map_w1, mode == 0 ? w1 : w0, (uint64_t)experts_local * N, (uint64_t)K, (uint64_t)K, 128)) return 3;
@@ -560,7 +560,7 @@ int launch_moe_tiles8(const void* x, int64_t x_stride, int divisor, const int* t
     args.expert_base = expert_base; args.experts_local = experts_local;
     args.scale0 = s0; args.scale1 = mode == 0 ? s1 : s0;
     args.route_weight = route_weight; args.out = (bf16*)out;
-    args.N = N; args.K = K; args.mode = mode;
+    args.N = N; args.K = K; args.mode = mode; args.status = status;
     const int64_t most = (int64_t)ceil_div(N, mode == 0 ? 128 : 256) * tiles;
     GLMB_LAUNCH(moe_grouped_fp8w_kernel<true>, (int)(most < 148 ? most : 148), MG_TILE8_THREADS, MG_TILE8_SMEM_BYTES, stream, map_w0, map_w0, map_w1, args);
     return (int)cudaGetLastError();

@@ -621,10 +621,10 @@ class GlmMoeDsaModel:
             else:
                 tile_expert, tile_routes, n_tiles, tiles, rt = self._route_tiles(ws.topk_ids[:rows], E)
             native.moe_gateup_fp8(x, tk, tile_expert, tile_routes, n_tiles, tiles, rt, lw.exp_gate_bits, lw.exp_up_bits,
-                                  lw.exp_gate_scale, lw.exp_up_scale, ebase, ws.act)
+                                  lw.exp_gate_scale, lw.exp_up_scale, ebase, ws.act, status=self.peer.status_ptr)
             if not one_launch:
                 native.moe_down_fp8(ws.act, ws.topk_w, tile_expert, tile_routes, n_tiles, tiles, rt, lw.exp_down_bits, lw.exp_down_scale,
-                                    ebase, ws.dw)
+                                    ebase, ws.dw, status=self.peer.status_ptr)
         if decode:
             if forked is not None:
                 self._join(forked)

@@ -342,20 +342,20 @@ def set_moe_mma(enabled: int) -> None:
     lib().glmb_set_moe_mma(int(enabled))
 
 
-def moe_gateup_fp8(x, top_k, tile_expert, tile_routes, n_tiles, tiles, rt, wg, wu, sg, su, expert_base, act):
+def moe_gateup_fp8(x, top_k, tile_expert, tile_routes, n_tiles, tiles, rt, wg, wu, sg, su, expert_base, act, *, status=None):
     experts_local, I, H = wg.shape
     _check(
         lib().glmb_moe_gateup_fp8(_p(x), C.c_int64(x.stride(0)), top_k, _p(tile_expert), _p(tile_routes), _p(n_tiles), tiles, rt,
-                                  _p(wg), _p(wu), _p(sg), _p(su), expert_base, experts_local, I, H, _p(act), _stream()),
+                                  _p(wg), _p(wu), _p(sg), _p(su), expert_base, experts_local, I, H, _p(act), _p(status), _stream()),
         "moe_gateup_fp8",
     )
 
 
-def moe_down_fp8(act, route_weight, tile_expert, tile_routes, n_tiles, tiles, rt, wd, sd, expert_base, dw):
+def moe_down_fp8(act, route_weight, tile_expert, tile_routes, n_tiles, tiles, rt, wd, sd, expert_base, dw, *, status=None):
     experts_local, H, I = wd.shape
     _check(
         lib().glmb_moe_down_fp8(_p(act), _p(route_weight), _p(tile_expert), _p(tile_routes), _p(n_tiles), tiles, rt, _p(wd),
-                                _p(sd), expert_base, experts_local, I, H, _p(dw), _stream()),
+                                _p(sd), expert_base, experts_local, I, H, _p(dw), _p(status), _stream()),
         "moe_down_fp8",
     )
 

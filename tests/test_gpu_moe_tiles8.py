@@ -57,3 +57,33 @@ def test_tiles_of_eight_on_tcgen05(native_lib, rows, tk, E, ebase, el, H, I, ske
             size = (act[p].abs() @ dq[2][e].abs().T) * weight.reshape(-1)[p]
             # the sum may round to the neighbouring bf16 (a step is at most 2^-7 of the value), and its product with the weight is rounded (2^-8)
             assert bool(((dw[p] - want).abs() <= (2**-7 + 2**-8 + 2**-14) * want.abs() + I * 2.0**-24 * size).all()), p
+
+
+def test_a_lost_wait_has_the_runners_status_word(native_lib, monkeypatch):
+    """The kernels of the 8-route tiles give up their waits after a limit: both launches of a prefill chunk hand over the word that the host reads after it."""
+    from glm_tpu_b200.config.model import small_geometry
+    from glm_tpu_b200.ops import native
+    from glm_tpu_b200.runner.gpu_runner import build_runner
+
+    handed = []
+
+    class Seen:
+        def __getattr__(self, name):
+            fn = getattr(inner, name)
+            if name not in ("glmb_moe_gateup_fp8", "glmb_moe_down_fp8"):
+                return fn
+            return lambda *args: (handed.append((name, getattr(args[-2], "value", args[-2]))), fn(*args))[1]
+
+    prompt = torch.randint(0, small_geometry(4).vocab_size, (60,), generator=torch.Generator().manual_seed(1)).tolist()
+    runner = build_runner(small_geometry(4), world=1, rank=0, device="cuda:0", seed=0, context_capacity=512, lanes=1, use_graphs=False, prefill_chunk=64)
+    try:
+        runner.model.few_routes_limit = 1 << 20  # 8-route tiles, whatever the small model's count of experts
+        inner = native.lib()
+        monkeypatch.setattr(native, "_lib", Seen())
+        runner.open_lane(0)
+        runner.extend(0, prompt)
+    finally:
+        monkeypatch.setattr(native, "_lib", inner)
+        runner.close()
+    assert {name for name, _ in handed} == {"glmb_moe_gateup_fp8", "glmb_moe_down_fp8"}
+    assert all(word == runner.peer.status_ptr for _, word in handed)
