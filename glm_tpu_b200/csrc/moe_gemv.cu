@@ -237,21 +237,23 @@ int glmb_launch_moe_down_mma(const void* act, const float* route_weight, const i
                              cudaStream_t stream);
 // Tiles of eight routes on tcgen05 (moe_grouped_tcgen05.cu).
 bool moe_tiles8_takes(const void* x, int64_t x_stride, const void* w0, const void* w1, const void* out, const int* tile_routes, int tiles, int experts, int N, int K);
+GLMB_API int glmb_moe_tiles8_pays(int tiles, int experts, int N, int K, int mode);
 int launch_moe_tiles8(const void* x, int64_t x_stride, int divisor, const int* tile_expert, const int* tile_routes, const int* n_tiles, int tiles,
                       const void* w0, const void* w1, const float* s0, const float* s1, int expert_base, int experts_local, int N, int K, int mode,
                       const float* route_weight, void* out, uint32_t* status, cudaStream_t stream);
 static int g_moe_mma = 1;
 // The fp32-FMA kernels below serve the shapes the mma.sync kernels refuse (hidden size not a multiple of 64, intermediate not a
 // multiple of 16, unaligned rows: fixtures).  The switch exists so that the tests can run BOTH families on shapes both take
-// (tests/test_gpu_ops.py::test_routed_experts); nothing in the product turns it off.
-GLMB_API void glmb_set_moe_mma(int enabled) { g_moe_mma = enabled ? 1 : 0; }
+// (tests/test_gpu_ops.py::test_routed_experts), and the tiles of eight on tcgen05 on small shapes too (2); nothing in the product changes it.
+GLMB_API void glmb_set_moe_mma(int enabled) { g_moe_mma = enabled > 1 ? 2 : enabled ? 1 : 0; }
+static bool moe_tiles8(int tiles, int experts, int N, int K, int mode) { return g_moe_mma == 2 || (g_moe_mma && glmb_moe_tiles8_pays(tiles, experts, N, K, mode)); }
 
 // Routed gate/up for `tiles` tiles of `rt` routes (rt in {1, 8}).  H % 16 == 0.
 GLMB_API int glmb_moe_gateup_fp8(const void* x, int64_t xs, int top_k, const int* tile_expert, const int* tile_routes,
                                  const int* n_tiles, int tiles, int rt, const void* wg, const void* wu, const float* sg,
                                  const float* su, int expert_base, int experts_local, int I, int H, void* act, uint32_t* status, void* stream) {
     if ((H & 15) || tiles < 1) return 1;
-    if (g_moe_mma && rt == 8 && top_k > 0 && moe_tiles8_takes(x, xs, wg, wu, act, tile_routes, tiles, experts_local, I, H))
+    if (rt == 8 && top_k > 0 && moe_tiles8_takes(x, xs, wg, wu, act, tile_routes, tiles, experts_local, I, H) && moe_tiles8(tiles, experts_local, I, H, 0))
         return launch_moe_tiles8(x, xs, top_k, tile_expert, tile_routes, n_tiles, tiles, wg, wu, sg, su, expert_base, experts_local, I, H, 0, nullptr, act,
                                  status, (cudaStream_t)stream);
     if (g_moe_mma && (rt == 1 || rt == 8) && !(H & 63) && !(I & 15) && !(xs & 7))
@@ -275,7 +277,7 @@ GLMB_API int glmb_moe_down_fp8(const void* act, const float* route_weight, const
                                const int* n_tiles, int tiles, int rt, const void* wd, const float* sd, int expert_base,
                                int experts_local, int I, int H, void* dw, uint32_t* status, void* stream) {
     if ((I & 15) || tiles < 1) return 1;
-    if (g_moe_mma && rt == 8 && moe_tiles8_takes(act, I, wd, nullptr, dw, tile_routes, tiles, experts_local, H, I))
+    if (rt == 8 && moe_tiles8_takes(act, I, wd, nullptr, dw, tile_routes, tiles, experts_local, H, I) && moe_tiles8(tiles, experts_local, H, I, 1))
         return launch_moe_tiles8(act, I, 1, tile_expert, tile_routes, n_tiles, tiles, wd, nullptr, sd, nullptr, expert_base, experts_local, H, I, 1,
                                  route_weight, dw, status, (cudaStream_t)stream);
     if (g_moe_mma && (rt == 1 || rt == 8) && !(I & 63) && !(H & 15))

@@ -535,12 +535,27 @@ GLMB_API int glmb_moe_grouped_fp8w(const void* a_sorted, int sorted_rows, const 
 }
 
 // Tiles of eight routes (route_sort8), the weights as M: an expert's weights are read once for up to MG_TILE8_ROUTES routes, where a kernel with a tile per
-// CTA reads and decodes them for every eight.  Takes what it can address; with fewer than 512 columns the stretch of products is too short for its epilogue.
+// CTA reads and decodes them for every eight.  What it can take; with fewer than 512 columns the stretch of products is too short for its epilogue.
 // mode 0: act [routes, N] of x [rows, K], route p of row p / divisor; mode 1: dw [routes, N] of x = act [routes, K], times route_weight.
 bool moe_tiles8_takes(const void* x, int64_t x_stride, const void* w0, const void* w1, const void* out, const int* tile_routes, int tiles, int experts, int N, int K) {
     return tile_routes && tiles <= MG_LIST && experts <= 65536 && K >= 512 && !(K & 63) && N >= 256 && !(N & 15) && !(x_stride & 7) &&
            !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1) | reinterpret_cast<uintptr_t>(out)) & 15);
 }
+// Whether it is expected to be the faster form.  Small experts, and few of them, end before its start is over ([8 x 1024 x 1024] and back, 9 rows of the top 2:
+// 13.1 + 12.1 us against 6.0 + 4.0 on mma.sync), and a round of its 148 CTAs just begun costs as much as a full one ([256 x 256 x 6144], 12 rows of the top 8: 84
+// against 67).  Here 10 us, and a round of items of 256 weight rows at 41 GB/s a CTA; there 3 us, and CTAs of 16 rows whose warps take chunks of 64 columns in
+// turns of eight (the form for up to 512 columns: a warp to 16 rows).  `tiles` is an eighth of the routes and one per expert (the length of the list, not its
+// count on the device); routes are taken to be dealt at random.  Of 231 measured launches (8 to 256 experts, 9 to 256 rows) the choice costs more than 9 % in three:
+// 64 rows of [16 x 640 x 576] 13.6 us, not 11.2, and of the second half 200 rows of [8 x 1024 x 1024] 19.4, not 16.0, 100 of [16 x 4096 x 1024] 35.7, not 30.9.
+static bool moe_tiles8_pays(int tiles, int experts, int N, int K, int mode) {
+    const double routes = 8.0 * (tiles > experts ? tiles - experts : 0) + 4.0, chosen = experts * (1.0 - pow(1.0 - 1.0 / experts, routes));
+    const double tiles8 = fmax(chosen, routes / 8 + chosen * 7 / 16), pieces = fmax(chosen, routes / MG_TILE8_ROUTES + chosen * 63 / 128);
+    const double rounds = pieces * ceil_div(N, mode == 0 ? 128 : 256) / 148, columns = ceil_div(K, 512) * 512.0 * (mode == 0 ? 2 : 1);
+    const double here = 10.0 + (rounds > 1.0 ? rounds + 0.5 : 1.0) * (256.0 * K / 41e3 + 1.25);
+    const double there = 3.0 + tiles8 * N / 16 * (0.8e-3 + 3.8e-6 * columns) * (mode == 1 && K <= 512 ? 0.75 : 1.0);
+    return here < there;
+}
+GLMB_API int glmb_moe_tiles8_pays(int tiles, int experts, int N, int K, int mode) { return experts > 0 && moe_tiles8_pays(tiles, experts, N, K, mode); }
 int launch_moe_tiles8(const void* x, int64_t x_stride, int divisor, const int* tile_expert, const int* tile_routes, const int* n_tiles, int tiles,
                       const void* w0, const void* w1, const float* s0, const float* s1, int expert_base, int experts_local, int N, int K, int mode,
                       const float* route_weight, void* out, uint32_t* status, cudaStream_t stream) {

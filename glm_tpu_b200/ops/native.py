@@ -338,8 +338,14 @@ def set_moe_experts_total(experts: int) -> None:
 
 
 def set_moe_mma(enabled: int) -> None:
-    """1 (default): FP8 expert GEMVs feed mma.sync; 0: the fp32-FMA kernels."""
+    """1 (default): FP8 expert GEMVs feed mma.sync, or tcgen05 where 8-route tiles pay; 0: the fp32-FMA kernels; 2: tcgen05 wherever 8-route tiles can."""
     lib().glmb_set_moe_mma(int(enabled))
+
+
+def moe_tiles8_pays(tiles: int, experts: int, N: int, K: int, mode: int) -> bool:
+    """Whether tcgen05 is the faster form of a launch over 8-route tiles (``tiles`` = routes // 8 + experts; mode 0: gate/up, 1: down)."""
+    lib()
+    return bool(_lib.glmb_moe_tiles8_pays(tiles, experts, N, K, mode))  # not a launch: past the wrapper that times launches
 
 
 def moe_gateup_fp8(x, top_k, tile_expert, tile_routes, n_tiles, tiles, rt, wg, wu, sg, su, expert_base, act, *, status=None):

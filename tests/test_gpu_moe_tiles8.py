@@ -59,6 +59,22 @@ def test_tiles_of_eight_on_tcgen05(native_lib, rows, tk, E, ebase, el, H, I, ske
             assert bool(((dw[p] - want).abs() <= (2**-7 + 2**-8 + 2**-14) * want.abs() + I * 2.0**-24 * size).all()), p
 
 
+# the shapes above are small: left to its rule the library takes mma.sync for some of them
+@pytest.mark.parametrize("case", test_tiles_of_eight_on_tcgen05.pytestmark[0].args[1])
+def test_tiles_of_eight_wherever_they_can(native_lib, case):
+    class Forced:
+        def __getattr__(self, name):
+            return getattr(native_lib, name)
+
+        def set_moe_mma(self, enabled):
+            native_lib.set_moe_mma(2 if enabled else 0)
+
+    try:
+        test_tiles_of_eight_on_tcgen05(Forced(), *case)
+    finally:
+        native_lib.set_moe_mma(1)
+
+
 def test_a_lost_wait_has_the_runners_status_word(native_lib, monkeypatch):
     """The kernels of the 8-route tiles give up their waits after a limit: both launches of a prefill chunk hand over the word that the host reads after it."""
     from glm_tpu_b200.config.model import small_geometry
