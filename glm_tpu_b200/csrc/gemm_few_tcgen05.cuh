@@ -1,6 +1,6 @@
 // Dense bf16 GEMM of few rows (a short prompt, the tail of a long one), included by gemm_tcgen05.cu:  C[rows, N] = A[rows, K] . B[N, K]^T.
 //
-// The WEIGHT rows are the M of the product (128 at a time, always full) and the activation rows its N, in steps of 16 up to 256; more rows
+// The WEIGHT rows are the M of the product (128 at a time, always full) and the activation rows its N, in steps of 16 up to 128; more rows
 // form several blocks.  A tile's K is dealt to the CTAs of a cluster, so that a projection with a few dozen tiles still has every SM streaming
 // weights; the partial tiles meet in distributed shared memory and are added in the order of K, the same sums in every run.
 //
@@ -55,7 +55,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int n0 = (tile % p.tiles_n) * 128, r0 = (tile / p.tiles_n) * p.n_box, rows = min(p.n_box, p.rows - r0);
     const int kblocks = (p.K + 63) / 64, per = (kblocks + p.splits - 1) / p.splits, k_first = split * per, steps = min(per, kblocks - k_first);  // >= 1
     const uint32_t stage_bytes = GF_A_BYTES + p.n_box * 128;
-    const uint32_t columns = p.n_box <= 32 ? 32 : p.n_box <= 64 ? 64 : p.n_box <= 128 ? 128 : 256;
+    const uint32_t columns = p.n_box <= 32 ? 32 : p.n_box <= 64 ? 64 : 128;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
@@ -172,7 +172,7 @@ struct GemmFewPlan { int n_box, blocks, splits, stages; double us; };
 
 // How K is dealt, by the time expected of a launch of its own: 13 us, a 64-wide step of 0.29 us and 0.11 more with 128 rows (a CTA alone on its SM; beyond
 // 148 CTAs they share the bandwidth), and 3 us to add 128 rows up over the cluster.  Measured against: [60 x 4096], K 18432, 1 to 8 splits: 92, 53, 41,
-// 37, 37, 36 us, expected 111, 64, 48, 40, 39, 38; [120 x 2048], K 6144: 49, 31, 25, 23, 21, 23, expected 51, 35, 29, 25, 22, 21.
+// 37, 37, 36 us, expected 112, 64, 48, 39, 36, 36; [120 x 2048], K 6144: 49, 31, 25, 23, 21, 23, expected 51, 35, 29, 25, 22, 21.
 // splits: 0: chosen.
 static GemmFewPlan gemm_few_plan(int rows, int N, int K, int splits = 0) {
     GemmFewPlan best = {0, 0, 0, 0, 1e30};

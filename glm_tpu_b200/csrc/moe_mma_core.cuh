@@ -27,16 +27,10 @@ __device__ __forceinline__ uint32_t dec2_packed(uint32_t two_codes, float scale)
 }
 
 // One 64-wide k chunk of one 16-row weight panel against the activation fragment xv (16 k values of route g).
-template <bool PACKED = false>
 __device__ __forceinline__ void chunk_mma(float (&acc)[4], const uint4& w_lo, const uint4& w_hi, float scale, const uint4& x0, const uint4& x1) {
     const uint32_t wl[4] = {w_lo.x, w_lo.y, w_lo.z, w_lo.w}, wh[4] = {w_hi.x, w_hi.y, w_hi.z, w_hi.w};
     const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if constexpr (PACKED)
-            mma_16816(acc, dec2_packed(wl[j] & 0xffffu, scale), dec2_packed(wh[j] & 0xffffu, scale), dec2_packed(wl[j] >> 16, scale), dec2_packed(wh[j] >> 16, scale),
-                      xw[2 * j], xw[2 * j + 1]);
-        else
-            mma_16816(acc, dec2(wl[j] & 0xffffu, scale), dec2(wh[j] & 0xffffu, scale), dec2(wl[j] >> 16, scale), dec2(wh[j] >> 16, scale), xw[2 * j], xw[2 * j + 1]);
-    }
+    for (int j = 0; j < 4; ++j)
+        mma_16816(acc, dec2(wl[j] & 0xffffu, scale), dec2(wh[j] & 0xffffu, scale), dec2(wl[j] >> 16, scale), dec2(wh[j] >> 16, scale), xw[2 * j], xw[2 * j + 1]);
 }

@@ -594,8 +594,9 @@ class GlmMoeDsaModel:
             self.trace.setdefault("topk_w", {})[layer] = ws.topk_w[:rows].clone()
         sort_kernel = self.route_sort_kernel and el <= 256 and ws.topk_ids[:rows].is_contiguous()
         # Chunks of up to 256 rows keep tiles of eight routes, as their launch program is recorded; behind those entry points lies the same kernel as
-        # behind the grouped form, which gathers the rows itself (no copy in expert order: 200 rows 1,131 + 620 us a layer of 256 experts).  Longer
-        # chunks sort into tiles of 128 routes: 300 rows 967 + 504 us, on mma.sync tiles of eight 1,867 + 1,233.
+        # behind the grouped form, which gathers the rows itself (no copy in expert order: 200 rows 1,131 + 620 us a layer of 256 experts, all of them
+        # chosen), or mma.sync where experts are small.  Longer chunks sort into tiles of 128 routes: 300 rows 967 + 504 us, on mma.sync tiles of eight
+        # 1,867 + 1,233 (with the experts that a prompt chooses, about 200).
         short = self.few_routes_rows is None or rows <= self.few_routes_rows
         few_per_expert = self.few_routes_gemv and sort_kernel and short and rows * tk < self.few_routes_limit * E
         if not decode and not few_per_expert and rows * tk >= 128 and H % 16 == 0 and I % 16 == 0:
