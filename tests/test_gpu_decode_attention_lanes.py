@@ -15,6 +15,13 @@ def test_several_lanes(native_lib, shape):
     single.test_decode_attention(native_lib, shape, False)
 
 
+# six rows on long rings: two parts of the keys to a CTA (eight key heads, also padded ones), splits by the rows (nine and twenty heads, values of 64, wide heads)
+@pytest.mark.parametrize("shape", [(32, 8, 128, 128, 3000, 4096), (16, 8, 96, 80, 2049, 4096), (80, 8, 128, 112, 2100, 4096), (18, 9, 128, 128, 2500, 4096),
+                                   (20, 20, 64, 128, 2200, 4096), (20, 20, 64, 64, 2200, 4096), (9, 9, 256, 200, 2100, 4096)])
+def test_several_lanes_on_long_rings(native_lib, shape):
+    single.test_decode_attention(native_lib, shape, False)
+
+
 @pytest.mark.parametrize("H,G,dim", [(32, 8, 128), (32, 8, 64), (16, 16, 128)])
 def test_a_rows_bits_do_not_depend_on_the_others(native_lib, H, G, dim):
     lanes, ring, positions = 8, 1024, [1000, 5, 517, 63, 64, 1023, 200, 900]
